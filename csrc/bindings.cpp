@@ -23,6 +23,8 @@ namespace py = pybind11;
 namespace msccl {
 cudaError_t launch_exec(const ExecArgs& args, int dtype, int proto, int width, int grid, cudaStream_t stream, bool cooperative);
 int max_coresident_ctas(int dtype, int proto, int width);
+cudaError_t launch_exec_one_gpu(const OneGpuArgs& args, int dtype, int proto, int width, int tbs, cudaStream_t stream, bool cooperative);
+int max_coresident_one_gpu(int dtype, int proto, int width);
 cudaError_t launch_twoshot_allreduce(char* const* heap_bases, char* mc_base, long long offset, long long bytes, int dtype,
                                      int rank, int nranks, SyncPage* const* syncs, unsigned long long timeout_ns, int ctas,
                                      cudaStream_t stream, void* rs_out, bool pipelined);
@@ -134,6 +136,35 @@ void launch(uintptr_t tbs, uintptr_t steps, uintptr_t ranks, const std::vector<l
            "launch of the MSCCL-IR executor kernel");
 }
 
+// One launch of the one-GPU interpreter.  `table` is the packed array of RankCtx (one per rank), copied into the kernel's
+// parameters; chunk / slice / tile are element counts, `slot` the bytes of a slice's FIFO slot.
+void launch_one_gpu(uintptr_t tbs, uintptr_t steps, const py::bytes& table, long long chunk, long long slice, long long tile,
+                    long long slot, int slices, int num_tbs, int dtype, int proto, int width, unsigned long long timeout_ns,
+                    int direct_mask, uintptr_t stream, bool cooperative, uintptr_t trace, int trace_steps) {
+  char* raw = nullptr;
+  Py_ssize_t bytes = 0;
+  if (PyBytes_AsStringAndSize(table.ptr(), &raw, &bytes) != 0) throw py::error_already_set();
+  msccl::OneGpuArgs a;
+  if (bytes <= 0 || bytes % sizeof(msccl::RankCtx) != 0 || static_cast<size_t>(bytes) > sizeof(a.ranks))
+    throw std::runtime_error("launch_one_gpu: bad rank table");
+  if (slices < 1 || tile < 1 || slice < 1) throw std::runtime_error("launch_one_gpu: bad geometry");
+  std::memset(&a, 0, sizeof(a));
+  std::memcpy(a.ranks, raw, static_cast<size_t>(bytes));
+  a.tbs = reinterpret_cast<const msccl::DevTb*>(tbs);
+  a.steps = reinterpret_cast<const msccl::DevStep*>(steps);
+  a.chunk_elems = chunk;
+  a.slice_elems = slice;
+  a.tile_elems = tile;
+  a.slot_bytes = slot;
+  a.timeout_ns = timeout_ns;
+  a.trace = reinterpret_cast<unsigned long long*>(trace);
+  a.trace_steps = trace_steps;
+  a.slices = slices;
+  a.direct_mask = direct_mask;
+  check_rt(msccl::launch_exec_one_gpu(a, dtype, proto, width, num_tbs, as_stream(stream), cooperative),
+           "launch of the one-GPU MSCCL-IR executor kernel");
+}
+
 py::dict layout() {
   py::dict d;
   d["sizeof_SyncPage"] = sizeof(SyncPage);
@@ -203,6 +234,8 @@ PYBIND11_MODULE(_msccl_native, m) {
         py::arg("elems") = std::vector<long long>(), py::arg("peer_heaps") = std::vector<uintptr_t>(),
         py::arg("sym_off") = std::vector<long long>(), py::arg("direct_mask") = 0, py::arg("epoch_base") = 0ull,
         py::arg("trace") = 0, py::arg("trace_steps") = 0, py::arg("wait_mode") = 0);
+  m.def("launch_one_gpu", &launch_one_gpu);
+  m.def("max_coresident_one_gpu", &msccl::max_coresident_one_gpu);
   m.def("max_coresident_ctas", &msccl::max_coresident_ctas);
 
   m.def("vmm_granularity", &msccl::vmm_granularity);

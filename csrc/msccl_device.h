@@ -71,6 +71,8 @@ struct alignas(128) SyncPage {
 enum StepFlags : uint8_t {
   SF_DIRECT_SEND = 1,   // the receiver's slot is (rbuf, roff) on the peer
   SF_DIRECT_RECV = 2,   // this receive may find its data already stored in (dstbuf, dstoff)
+  SF_DIRECT_ALWAYS = 4, // nothing on the receiving GPU touches the slots of this connection before their receives: when all
+                        // ranks run in one kernel the sender need not ask (exec_one_gpu.cu)
 };
 
 struct alignas(16) DevStep {    // 32 bytes, copied as two 16-byte vectors
@@ -138,6 +140,22 @@ struct ExecArgs {
   // barrier that ends the step) and signalling; the sixth word is spare.
   unsigned long long* trace;
   int trace_steps;            // steps per threadblock the trace has room for
+};
+
+// Launch of the one-GPU interpreter (exec_one_gpu.cu): every rank on this device, each threadblock run by `slices` CTAs.
+struct OneGpuArgs {
+  const DevTb* tbs;
+  const DevStep* steps;
+  long long chunk_elems;      // elements per chunk
+  long long slice_elems;      // elements of each chunk that one CTA of a threadblock works on (the last may have fewer)
+  long long tile_elems;       // elements of a slice processed per iteration
+  long long slot_bytes;       // FIFO slot of one slice
+  unsigned long long timeout_ns;
+  unsigned long long* trace;  // as in ExecArgs; slice 0 of every threadblock records
+  int trace_steps;
+  int slices;
+  int direct_mask;
+  RankCtx ranks[kMaxRanks];
 };
 
 static_assert(sizeof(DevStep) == 32 && sizeof(DevTb) == 64, "layout shared with msccl/runtime/plan.py");

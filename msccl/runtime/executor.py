@@ -24,8 +24,8 @@ import os
 import torch
 
 from msccl.runtime.comm import Communicator
-from msccl.runtime.plan import (HostPlan, PlanError, access_width, chunk_geometry, compile_plan, tile_geometry,
-                                K_FIFO_SLOTS)
+from msccl.runtime.plan import (HostPlan, PlanError, access_width, chunk_geometry, compile_plan, fold_reduce_chains,
+                                one_gpu_geometry, tile_geometry, K_FIFO_SLOTS)
 from msccl.xml.loader import AlgoIR, load_plan_table, load_xml
 
 DTYPE_CODES = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
@@ -57,7 +57,10 @@ class DevicePlan:
         self.slot_bytes = slot // 1024 * 1024
         if self.slot_bytes < 1024:
             raise PlanError('FIFO area too small for this program')
-        self.host: HostPlan = compile_plan(algo, comm.local_ranks, self.slot_bytes)
+        # with every rank on this GPU a hop between threadblocks costs more than the add it passes on
+        self.host: HostPlan = compile_plan(fold_reduce_chains(algo) if comm.emulated_mode else algo, comm.local_ranks,
+                                           self.slot_bytes)
+        self.geometry = {}         # emulated mode: (chunk elements, element size, width, proto) -> launch geometry
         nat = comm.native
         self.dev_tbs = nat.upload(self.host.tb_bytes)
         self.dev_steps = nat.upload(self.host.step_bytes)
@@ -81,7 +84,6 @@ class Executor:
         # guarantees co-residency).  MSCCL_EXEC_COOPERATIVE=0 is a diagnostic switch for an otherwise idle GPU.
         self.cooperative = os.environ.get('MSCCL_EXEC_COOPERATIVE', '1') != '0'
         self.last_algorithm = None  # what the last collective call dispatched to
-        self._ctx_cache = {}       # emulated mode: buffer pointers of all ranks -> device copy of the rank table
         self.last_direct_mask = 0  # buffers (bit 0 input, 1 output, 2 scratch) the last run() stored into directly
         self._trace = None
         # how the warps of a CTA learn that a step may start: 'poll' shared memory, or at a CTA 'barrier'
@@ -196,34 +198,32 @@ class Executor:
         proto = plan.host.proto
         if proto == 2 and width != 16:
             proto = 1                         # LL128 lines need 16-byte chunks; such calls run on the LL packets
-        tile, iterations = tile_geometry(plan.host, chunk, esize, plan.slot_bytes, width, proto)
+        if not comm.emulated_mode:
+            tile, iterations = tile_geometry(plan.host, chunk, esize, plan.slot_bytes, width, proto)
         stream_h = (stream or torch.cuda.current_stream()).cuda_stream
         nat = comm.native
         key = (DTYPE_CODES[dtype], proto, width)
         if key not in self._checked_grid:
-            self._checked_grid[key] = nat.max_coresident_ctas(*key)
+            self._checked_grid[key] = (nat.max_coresident_one_gpu if comm.emulated_mode else nat.max_coresident_ctas)(*key)
         if plan.grid > self._checked_grid[key]:
             raise PlanError(f'{plan.grid} threadblocks cannot be co-resident on this device '
                             f'(limit {self._checked_grid[key]})')
         trace_ptr, trace_steps = 0, 0
         if trace:
-            trace_steps = max(1, max(len(tb.steps) for g in algo.gpus for tb in g.tbs))
+            trace_steps = max(1, max(len(tb.steps) for g in plan.host.algo.gpus for tb in g.tbs))
             self._trace = torch.zeros(plan.grid * trace_steps * 6, dtype=torch.int64, device=first.device)
             self._trace_shape = (plan, trace_steps)
             trace_ptr = self._trace.data_ptr()
-        geom = [chunk, tile, plan.slot_bytes, iterations, comm.world, 0, plan.grid, key[0], proto, width]
         if comm.emulated_mode:
-            # the per-rank buffer table lives on the device, one copy per distinct set of buffers: a
-            # host-to-device copy per launch would queue behind any large input copy in flight
-            table = tuple(buffers[r] + sizes[r] for r in comm.local_ranks)
-            rankctx = self._ctx_cache.get(table)
-            if rankctx is None:
-                if len(self._ctx_cache) >= 64:
-                    nat.device_free(self._ctx_cache.pop(next(iter(self._ctx_cache))))
-                rankctx = self._ctx_cache[table] = nat.upload(comm.rankctx_bytes(buffers, sizes))
+            geometry = plan.geometry.get((chunk, esize, width, proto))
+            if geometry is None:
+                geometry = plan.geometry[(chunk, esize, width, proto)] = one_gpu_geometry(
+                    plan.host, chunk, esize, plan.slot_bytes, width, proto, self._checked_grid[key])
+            slices, slice_elems, tile, slot = geometry
             self.last_direct_mask = 7 if direct else 0
-            nat.launch(plan.dev_tbs, plan.dev_steps, rankctx, geom, comm.timeout_ns, stream_h, self.cooperative,
-                       direct_mask=self.last_direct_mask, trace=trace_ptr, trace_steps=trace_steps, wait_mode=self.wait_mode)
+            nat.launch_one_gpu(plan.dev_tbs, plan.dev_steps, comm.rankctx_bytes(buffers, sizes), chunk, slice_elems, tile, slot,
+                               slices, plan.grid, key[0], proto, width, comm.timeout_ns, self.last_direct_mask, stream_h,
+                               self.cooperative, trace_ptr, trace_steps)
         else:
             r = comm.rank
             sym_off, mask = [-1, -1, -1], 0
@@ -233,6 +233,7 @@ class Executor:
                     if off is not None:
                         sym_off[b], mask = off, mask | (1 << b)
             self.last_direct_mask = mask
+            geom = [chunk, tile, plan.slot_bytes, iterations, comm.world, 0, plan.grid, key[0], proto, width]
             nat.launch(plan.dev_tbs, plan.dev_steps, comm.dev_rankctx, geom, comm.timeout_ns, stream_h, self.cooperative,
                        bufs=list(buffers[r]), elems=list(sizes[r]), peer_heaps=list(comm.heap_ptrs), sym_off=sym_off,
                        direct_mask=mask, trace=trace_ptr, trace_steps=trace_steps, wait_mode=self.wait_mode)
@@ -269,7 +270,7 @@ class Executor:
         origin = int(starts.min()) if starts.numel() else 0
         rows, cta = [], 0
         for r in self.comm.local_ranks:
-            for tb in plan.algo.gpus[r].tbs:
+            for tb in plan.host.algo.gpus[r].tbs:
                 for si, st in enumerate(tb.steps):
                     t0, t1, wait, move, signal, _ = (int(v) for v in raw[cta, si])
                     if t1 or t0:

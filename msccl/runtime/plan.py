@@ -19,7 +19,8 @@ Besides the translation, three analyses run here:
   dependencies, reference ``msccl/language/ir.py:264-291``) becomes one multi-input add with one store.
 """
 import struct
-from dataclasses import dataclass, field
+from collections import Counter
+from dataclasses import dataclass, field, replace
 from typing import Dict, List
 
 from msccl.xml.loader import AlgoIR
@@ -35,7 +36,7 @@ K_FIFO_SLOTS = 4
 K_MAX_BATCH = 8                 # `re` steps fused into one pass (csrc/msccl_device.h kMaxBatch)
 K_MAX_STEPS_PER_TB = 4094       # the progress word keeps 12 bits of step + 1 ...
 K_MAX_ITERATIONS = 1 << 20      # ... and 20 bits of iteration
-SF_DIRECT_SEND, SF_DIRECT_RECV = 1, 2
+SF_DIRECT_SEND, SF_DIRECT_RECV, SF_DIRECT_ALWAYS = 1, 2, 4
 _TB = struct.Struct('<4h4i2i2q4i')
 _STEP = struct.Struct('<4B2h3i4Bi2H')
 assert _TB.size == 64 and _STEP.size == 32
@@ -217,6 +218,120 @@ def _batches(tb):
     return out
 
 
+def _overlap(o1, c1, o2, c2):
+    return o1 < o2 + c2 and o2 < o1 + c1
+
+
+def _find_chain(algo, gpu, waiters, limit):
+    """A chain of ``re`` steps into one slot, each in another threadblock and waiting for the one before, that may run as
+    one multi-input add at the place of the last one.  Returns ``[(tb, step), ...]`` or None.
+
+    A link may be taken out of its threadblock when nobody but the next link waits for it and whatever follows it in
+    its threadblock already waits for the end of the chain: then everything that was ordered after a link is ordered
+    after the end, and everything that came before a link is waited for by the end."""
+    def slot(st, src):
+        return algo.resolve(gpu.id, st.srcbuf, st.srcoff) if src else algo.resolve(gpu.id, st.dstbuf, st.dstoff)
+
+    for t, tb in enumerate(gpu.tbs):
+        for i, st in enumerate(tb.steps):
+            if st.type != 're' or (i + 1 < len(tb.steps) and tb.steps[i + 1].type == 're'):
+                continue
+            if any(x.type == 're' and x.depid == t and x.deps == i and slot(x, False) == slot(st, False) and
+                   not (j + 1 < len(other.steps) and other.steps[j + 1].type == 're')
+                   for o, other in enumerate(gpu.tbs) if o != t for j, x in enumerate(other.steps)):
+                continue                                    # not the end of its chain
+            chain = [(t, i)]
+            while len(chain) < limit:
+                ct, ci = chain[0]
+                cur = gpu.tbs[ct].steps[ci]
+                if ci > 0 and gpu.tbs[ct].steps[ci - 1].type == 're':
+                    break
+                if not 0 <= cur.depid < len(gpu.tbs) or cur.depid in [x for x, _ in chain]:
+                    break
+                prev_tb = gpu.tbs[cur.depid]
+                if not 0 <= cur.deps < len(prev_tb.steps):
+                    break
+                prev = prev_tb.steps[cur.deps]
+                if (prev.type != 're' or slot(prev, False) != slot(st, False) or prev.cnt != st.cnt or
+                        waiters[(cur.depid, cur.deps)] != 1 or
+                        (cur.deps > 0 and prev_tb.steps[cur.deps - 1].type == 're')):
+                    break
+                if cur.deps + 1 < len(prev_tb.steps):
+                    behind = prev_tb.steps[cur.deps + 1]
+                    if behind.depid != t or behind.deps < i:
+                        break
+                chain.insert(0, (cur.depid, cur.deps))
+            dst = slot(st, False)
+            srcs = [slot(gpu.tbs[ct].steps[ci], True) for ct, ci in chain]
+            if any(b == dst[0] and _overlap(o, st.cnt, dst[1], st.cnt) for b, o in srcs):
+                continue
+            if len(chain) > 1:
+                return chain
+    return None
+
+
+def fold_reduce_chains(algo: AlgoIR) -> AlgoIR:
+    """The program with chains of local reduces that pass a slot from threadblock to threadblock (n - 1 hops of store,
+    fence, flag and poll in the one-shot and two-shot all-reduce) replaced by one multi-input add at the end of the chain
+    - same operands, same order, same roundings.  The input is not modified."""
+    gpus, changed = [], False
+    for g in algo.gpus:
+        gpu = replace(g, tbs=[replace(tb, steps=[replace(st) for st in tb.steps]) for tb in g.tbs])
+        gpus.append(gpu)
+        if any(tb.id != i for i, tb in enumerate(gpu.tbs)):
+            continue
+        while True:
+            waiters = Counter((st.depid, st.deps) for tb in gpu.tbs for st in tb.steps if st.depid >= 0)
+            chain = _find_chain(algo, gpu, waiters, K_MAX_BATCH)
+            if chain is None:
+                break
+            changed = True
+            last_t, last_i = chain[-1]
+            removed = {t: set() for t, _ in chain}
+            head, adds = {}, []          # tb -> latest step that must be done before the first add; the adds in chain order
+            for k, (t, i) in enumerate(chain):
+                steps = gpu.tbs[t].steps
+                removed[t].add(i)
+                deps = [steps[i]] if k == 0 else []
+                j = i - 1
+                while j >= 0 and steps[j].type == 'nop' and waiters[(t, j)] == 0 and not steps[j].hasdep:
+                    deps.append(steps[j])
+                    removed[t].add(j)
+                    j -= 1
+                for st in deps:
+                    if st.depid >= 0 and st.depid != last_t:
+                        head[st.depid] = max(head.get(st.depid, -1), st.deps)
+                add = replace(steps[i], depid=-1, deps=-1, hasdep=False)
+                if t != last_t and j >= 0:                  # what came before the link fills its source
+                    steps[j].hasdep = True
+                    add.depid, add.deps = t, j
+                adds.append(add)
+            for add in adds:
+                if add.depid in head:                       # one wait per threadblock, the later of the two
+                    head[add.depid] = max(head[add.depid], add.deps)
+                    add.depid = add.deps = -1
+            hasdep = gpu.tbs[last_t].steps[last_i].hasdep
+            group = [replace(adds[0], type='nop', srcbuf='i', srcoff=-1, dstbuf='o', dstoff=-1, cnt=0, depid=d, deps=s)
+                     for d, s in sorted(head.items())] + adds
+            group[-1].hasdep = hasdep
+            renumber = {}
+            for t in removed:
+                fresh = []
+                for i, st in enumerate(gpu.tbs[t].steps):
+                    if (t, i) == (last_t, last_i):
+                        fresh.extend(group)
+                    elif i not in removed[t]:
+                        fresh.append(st)
+                    renumber[(t, i)] = len(fresh) - 1
+                gpu.tbs[t].steps = fresh
+            for tb in gpu.tbs:
+                for i, st in enumerate(tb.steps):
+                    st.s = i
+                    if (st.depid, st.deps) in renumber:
+                        st.deps = renumber[(st.depid, st.deps)]
+    return replace(algo, gpus=gpus) if changed else algo
+
+
 def compile_plan(algo: AlgoIR, local_ranks, slot_bytes: int, check=True, direct=True, batch=True) -> HostPlan:
     if check:
         problems = validate(algo)
@@ -288,6 +403,8 @@ def compile_plan(algo: AlgoIR, local_ranks, slot_bytes: int, check=True, direct=
                         if other.type in ('r', 'rcs') and other.cnt == st.cnt:
                             pb, po = algo.resolve(pr, other.dstbuf, other.dstoff)
                             flags |= SF_DIRECT_SEND
+                            if opens[(pr, pt)][0] == opens[(pr, pt)][3]:
+                                flags |= SF_DIRECT_ALWAYS
                             rbuf, roff = BUF_CODES[pb], po
                             plan.direct_bufs[pr].add(pb)
                             plan.direct_steps += 1
@@ -331,6 +448,48 @@ def access_width(chunk_elems: int, elem_size: int, pointers=()):
     if (chunk_elems * elem_size) % 16 == 0 and all(p % 16 == 0 for p in pointers):
         return 16
     return elem_size
+
+
+# One-GPU interpreter (csrc/exec_one_gpu.cu).  SLICE_BYTES: a CTA's share of a chunk below which another slice only adds
+# flags.  TILE_BYTES: what a CTA moves between two signals of the Simple protocol.
+ONE_GPU_SLICE_BYTES = 4 << 10
+ONE_GPU_TILE_BYTES = 128 << 10
+
+
+def one_gpu_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_bytes: int, width: int, proto: int, max_ctas: int):
+    """(slices, slice_elems, tile_elems, slice_slot_bytes) of a launch with every rank on one GPU.
+
+    Each chunk is cut into ``slices`` parts of ``slice_elems`` elements (whole 128-byte lines), one CTA of every threadblock
+    per part: as many as fit on the GPU at once, have flags of their own (channels x slices, threadblocks x slices) and
+    are worth a CTA.  A slice moves in tiles of ``tile_elems`` through FIFO slots of ``slice_slot_bytes``."""
+    per_access = width // elem_size
+    if (chunk_elems * elem_size) % width:
+        raise PlanError(f'chunks of {chunk_elems * elem_size} bytes are not whole {width}-byte accesses')
+    tbs = max(plan.total_tbs(), 1)
+    chans = 1 + max((tb.chan for g in plan.algo.gpus for tb in g.tbs), default=0)
+    fifo_bytes = {0: width, 1: 32 if width == 16 else 8, 2: 128}[proto]          # one access (LL128: one line) in the FIFO
+    most = min(max_ctas // tbs, K_MAX_CHANNELS // chans, K_MAX_TBS // max(plan.algo.max_tbs_per_gpu(), 1),
+               slot_bytes // max(1024, 128 * -(-plan.max_cnt * fifo_bytes // 128)), -(-chunk_elems * elem_size // ONE_GPU_SLICE_BYTES))
+    slices = max(1, most)
+    line = max(per_access, 128 // elem_size)
+    slice_elems = -(-(-(-chunk_elems // slices)) // line) * line
+    slices = max(1, -(-chunk_elems // slice_elems))
+    slot = slot_bytes // slices // 128 * 128
+    if proto == 2:
+        tile = slot // 128 // plan.max_cnt * 15 // 2 * per_access                # 15 units of 8 bytes per line
+    else:
+        tile = slot // (plan.max_cnt * fifo_bytes) * per_access
+    if tile <= 0:
+        raise PlanError('FIFO slot too small for this program')
+    if proto == 0:
+        want = max(per_access, ONE_GPU_TILE_BYTES // plan.max_cnt // elem_size // line * line)
+        want = max(want, -(-slice_elems // (K_MAX_ITERATIONS - 1) // per_access + 1) * per_access)
+        tile = min(tile, want)
+    tile = min(tile, slice_elems)
+    if -(-slice_elems // tile) >= K_MAX_ITERATIONS:
+        raise PlanError(f'{-(-slice_elems // tile)} iterations through FIFO slots of {slot} bytes exceed the executor limit '
+                        f'of {K_MAX_ITERATIONS}: use a larger FIFO area')
+    return slices, slice_elems, tile, slot
 
 
 def tile_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_bytes: int, width: int = 16, proto=None):

@@ -1,0 +1,63 @@
+"""Host side of the one-GPU interpreter: folded reduce chains against the unfolded program, and its launch geometry."""
+import pytest
+import torch
+
+from msccl.interp import input_chunks_of, run_algorithm
+from msccl.language import MSCCLProgram, ThreadblockPolicy
+from msccl.language.collectives import AllReduce
+from msccl.programs.allreduce import allreduce_allpairs, allreduce_one_shot, allreduce_ring, allreduce_two_shot
+from msccl.runtime import plan as P
+from msccl.topologies import fully_connected
+from msccl.xml import load_xml
+from msccl.xml.validator import validate
+
+PROGRAMS = {'one_shot': (allreduce_one_shot, 1), 'two_shot': (allreduce_two_shot, None), 'ring': (lambda n: allreduce_ring(n, 2), None),
+            'allpairs': (allreduce_allpairs, 'square')}
+
+
+def _program(name, ranks, instances=1, **kw):
+    body, chunks = PROGRAMS[name]
+    chunks = ranks * ranks if chunks == 'square' else chunks or ranks
+    prog = MSCCLProgram(name, fully_connected(ranks), AllReduce(ranks, chunks, True), instances,
+                        threadblock_policy=ThreadblockPolicy.manual, **kw)
+    with prog:
+        body(ranks)
+    return load_xml(prog.generate_xml())
+
+
+@pytest.mark.parametrize('name,ranks,instances', [('one_shot', 2, 1), ('one_shot', 3, 2), ('one_shot', 8, 1), ('two_shot', 4, 1),
+                                                  ('two_shot', 8, 2), ('one_shot', 12, 1), ('ring', 4, 2), ('allpairs', 4, 1)])
+def test_folded_chains_round_like_the_program(name, ranks, instances):
+    # 12 ranks: eleven adds, more than one multi-input add takes
+    algo = _program(name, ranks, instances)
+    before = [[(st.type, st.depid, st.deps) for tb in g.tbs for st in tb.steps] for g in algo.gpus]
+    folded = P.fold_reduce_chains(algo)
+    assert [[(st.type, st.depid, st.deps) for tb in g.tbs for st in tb.steps] for g in algo.gpus] == before
+    assert validate(folded) == []
+    reduces = lambda a: sum(st.type == 're' for g in a.gpus for tb in g.tbs for st in tb.steps)   # noqa: E731
+    assert reduces(folded) == reduces(algo)
+    if name in ('one_shot', 'two_shot') and ranks > 2:
+        waits = lambda a: sum(st.type == 're' and a.gpus[0].tbs[st.depid].steps[st.deps].type == 're'    # noqa: E731
+                              for tb in a.gpus[0].tbs for st in tb.steps if st.depid >= 0)
+        assert waits(folded) <= (ranks - 1) // P.K_MAX_BATCH < waits(algo)
+    gen = torch.Generator().manual_seed(3)
+    host = [torch.randn(input_chunks_of(algo, r) * 24, generator=gen).bfloat16() for r in range(ranks)]
+    want = run_algorithm(algo, host, 24, dtype=torch.bfloat16)
+    got = run_algorithm(folded, host, 24, dtype=torch.bfloat16)
+    assert all(torch.equal(w.view(torch.int16), g.view(torch.int16)) for w, g in zip(want, got))
+
+
+@pytest.mark.parametrize('chunk,esize', [(1, 2), (7, 4), (8, 2), (333333, 2), (4096, 4), (1 << 22, 2), (5 * (1 << 20) + 8, 4)])
+@pytest.mark.parametrize('proto', [0, 1, 2])
+@pytest.mark.parametrize('max_ctas', [32, 148, 592])
+def test_one_gpu_geometry_covers_the_chunk(chunk, esize, proto, max_ctas):
+    plan = P.compile_plan(_program('two_shot', 4, 2, protocol='LL'), range(4), 64 << 10)
+    width = P.access_width(chunk, esize)
+    proto = 1 if proto == 2 and width != 16 else proto
+    slices, slice_elems, tile, slot = P.one_gpu_geometry(plan, chunk, esize, 64 << 10, width, proto, max_ctas)
+    assert slices * plan.total_tbs() <= max_ctas and (slices - 1) * slice_elems < chunk <= slices * slice_elems
+    assert slice_elems * esize % width == 0 and 0 < tile <= slice_elems and tile * esize % width == 0
+    assert slot % 128 == 0 and slot * slices <= 64 << 10
+    accesses = tile * esize // width
+    fifo = {0: accesses * width, 1: accesses * (32 if width == 16 else 8), 2: -(-2 * accesses // 15) * 128}[proto]
+    assert fifo * plan.max_cnt <= slot
