@@ -10,6 +10,7 @@
 #include <cstring>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "fused_tp.h"
@@ -136,30 +137,29 @@ void launch(uintptr_t tbs, uintptr_t steps, uintptr_t ranks, const std::vector<l
            "launch of the MSCCL-IR executor kernel");
 }
 
-// One launch of the one-GPU interpreter.  `table` is the packed array of RankCtx (one per rank), copied into the kernel's
-// parameters; chunk / slice / tile are element counts, `slot` the bytes of a slice's FIFO slot.
-void launch_one_gpu(uintptr_t tbs, uintptr_t steps, const py::bytes& table, long long chunk, long long slice, long long tile,
-                    long long slot, int slices, int num_tbs, int dtype, int proto, int width, unsigned long long timeout_ns,
-                    int direct_mask, uintptr_t stream, bool cooperative, uintptr_t trace, int trace_steps) {
+// One launch of the one-GPU interpreter.  `table` is the packed array of OneGpuRank (one per rank), copied into the kernel's
+// parameters; `geom` = (CTAs per threadblock, slices per CTA, elements of a slice, of a tile, bytes of a slice's FIFO slot).
+void launch_one_gpu(uintptr_t tbs, uintptr_t steps, const py::bytes& table, long long chunk,
+                    const std::tuple<int, int, long long, long long, long long>& geom, int num_tbs, int dtype, int proto, int width,
+                    unsigned long long timeout_ns, int direct_mask, uintptr_t stream, bool cooperative, uintptr_t trace,
+                    int trace_steps) {
   char* raw = nullptr;
   Py_ssize_t bytes = 0;
   if (PyBytes_AsStringAndSize(table.ptr(), &raw, &bytes) != 0) throw py::error_already_set();
   msccl::OneGpuArgs a;
-  if (bytes <= 0 || bytes % sizeof(msccl::RankCtx) != 0 || static_cast<size_t>(bytes) > sizeof(a.ranks))
+  if (bytes <= 0 || bytes % sizeof(msccl::OneGpuRank) != 0 || static_cast<size_t>(bytes) > sizeof(a.ranks))
     throw std::runtime_error("launch_one_gpu: bad rank table");
-  if (slices < 1 || tile < 1 || slice < 1) throw std::runtime_error("launch_one_gpu: bad geometry");
   std::memset(&a, 0, sizeof(a));
   std::memcpy(a.ranks, raw, static_cast<size_t>(bytes));
   a.tbs = reinterpret_cast<const msccl::DevTb*>(tbs);
   a.steps = reinterpret_cast<const msccl::DevStep*>(steps);
   a.chunk_elems = chunk;
-  a.slice_elems = slice;
-  a.tile_elems = tile;
-  a.slot_bytes = slot;
+  std::tie(a.ctas_per_tb, a.streams, a.slice_elems, a.tile_elems, a.slot_bytes) = geom;
+  if (a.ctas_per_tb < 1 || (a.streams != 1 && a.streams != 2 && a.streams != 4) || a.slice_elems < 1 || a.tile_elems < 1)
+    throw std::runtime_error("launch_one_gpu: bad geometry");
   a.timeout_ns = timeout_ns;
   a.trace = reinterpret_cast<unsigned long long*>(trace);
   a.trace_steps = trace_steps;
-  a.slices = slices;
   a.direct_mask = direct_mask;
   check_rt(msccl::launch_exec_one_gpu(a, dtype, proto, width, num_tbs, as_stream(stream), cooperative),
            "launch of the one-GPU MSCCL-IR executor kernel");
@@ -168,6 +168,9 @@ void launch_one_gpu(uintptr_t tbs, uintptr_t steps, const py::bytes& table, long
 py::dict layout() {
   py::dict d;
   d["sizeof_SyncPage"] = sizeof(SyncPage);
+  d["sizeof_OneGpuFlags"] = sizeof(msccl::OneGpuFlags);
+  d["kOneGpuChannels"] = msccl::kOneGpuChannels;
+  d["kOneGpuProgress"] = msccl::kOneGpuProgress;
   d["sizeof_DevStep"] = sizeof(msccl::DevStep);
   d["sizeof_DevTb"] = sizeof(msccl::DevTb);
   d["sizeof_RankCtx"] = sizeof(msccl::RankCtx);

@@ -2,21 +2,24 @@
 // exec_kernel.cu - steps of a threadblock in order, the program's protocol, FIFOs, credits, bounds checks, bounded
 // waits, bit-identical sums - but laid out for one device:
 //
-//   * Slices.  Every step works element by element, so a chunk is cut into K slices that never meet: K CTAs run one
-//     threadblock, each on its own slice, with its own FIFO slots, counters and progress word.  One CTA per SM (the
-//     layout of exec_kernel.cu) leaves the SMs of idle receivers empty and pays every flag round trip in full; four CTAs
-//     of 256 threads per SM hide them behind each other.
-//   * Roles.  Six data warps move; a control warp polls the flags of the next steps, one flag per lane, and hands
-//     the finished job (pointers, sizes) to the data warps; a signal warp fences and publishes what a step finished while
-//     the data warps are in the next one.  Jobs are double buffered: control runs up to two steps ahead.
+//   * Slices.  Every step works element by element, so a chunk is cut into slices that never meet, each with its own FIFO
+//     slots, counters and progress words.  K CTAs run one threadblock, and each of them runs P slices: while one slice
+//     waits for its tile to come round the ring, another moves.  One CTA per SM (the layout of exec_kernel.cu) leaves the
+//     SMs of idle receivers empty and pays every flag round trip in full.
+//   * Roles.  Six data warps move; a control warp polls the flags of its slices' next steps, one flag per lane, and hands
+//     jobs that are ready (pointers, sizes) to the data warps; a signal warp fences and publishes what a job finished while
+//     the data warps are in the next one.  Jobs are double buffered.  Slices share the data warps only under the Simple
+//     protocol: there a job never waits once it has been handed over (a flag-in-data job does, and could wait for one
+//     queued behind it).
+//   * Chunks that are not multiples of 16 bytes still move in 16-byte vectors: stores are aligned, loads are put together
+//     from two aligned vectors.
 //   * Scope.  All flags are read and written at GPU scope: a system-scope fence costs more and orders nothing extra here.
 //   * No drain: the FIFO contents cannot be wanted after the kernel's end, because every receiver is part of it.  No
 //     opening handshake for slots that nothing touches before their receive (SF_DIRECT_ALWAYS): every rank's earlier
 //     work on this GPU is done when the kernel runs.
 //   * The rank table travels in the kernel parameters: no device copy per set of buffers, nothing kept by address.
 //
-// Bound by L2 / HBM traffic from about 1 MB per chunk on, by the flag round trips (store, fence, poll: about 1.5 us a
-// hop) below.
+// Bound by L2 / HBM traffic from about 1 MB per chunk on, by the flag round trips (store, fence, poll) below.
 #include <cstdio>
 
 #include "exec_common.cuh"
@@ -47,8 +50,9 @@ struct __align__(16) Job {
   unsigned int flag_in, flag_out;
   unsigned long long flag_in128, flag_out128;
   // what the signal warp publishes
-  int fence, step, steps, iter;   // first step of the pass and how many (nops in front and batch members included)
+  int fence, traced, step, steps, iter;   // first step of the pass and how many (nops in front and batch members included)
   unsigned long long tail, credit, opened, progress;     // 0: nothing to publish
+  unsigned long long *tail_out, *credit_out, *open_out, *progress_out;
   unsigned long long t0, t1;      // trace
 };
 
@@ -56,6 +60,7 @@ struct Shared {
   Job job[2];
   unsigned long long go[2], done[2];     // mbarriers
   int fail;                              // a flag-in-data poll or a wait ran out of time
+  int leave;                             // the first data warp waited too long for a job: all leave
   int signalled;                         // passes the signal warp has finished with
   DevStep steps[kOgSmemSteps];
 };
@@ -108,6 +113,69 @@ __device__ __forceinline__ void og_move(const char* in0, const char* add1, char*
 #pragma unroll
       for (int u = 0; u < U; ++u)
         if (base + u * kOgData < n) Access<W>::st(out1 + static_cast<long long>(base + u * kOgData) * W, val[u]);
+    }
+  }
+}
+
+// ---- chunks that do not start on 16-byte boundaries ------------------------------------------------------------------
+// 16 bytes at any multiple of 2.  A second aligned vector is read only if it holds one of them.
+struct Unaligned {
+  uint4 lo, hi;
+  __device__ __forceinline__ void load(const char* p) {
+    const char* base = reinterpret_cast<const char*>(reinterpret_cast<unsigned long long>(p) & ~15ull);
+    lo = *reinterpret_cast<const uint4*>(base);
+    hi = base != p ? *reinterpret_cast<const uint4*>(base + 16) : lo;
+  }
+  __device__ __forceinline__ uint4 get(unsigned int shift) const {        // shift = address % 16
+    unsigned int w[7] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z};
+    unsigned int last = hi.w;
+    if (shift & 8u) { w[0] = w[2]; w[1] = w[3]; w[2] = w[4]; w[3] = w[5]; w[4] = w[6]; w[5] = last; }
+    if (shift & 4u) { w[0] = w[1]; w[1] = w[2]; w[2] = w[3]; w[3] = w[4]; w[4] = w[5]; }
+    if (shift & 2u) return make_uint4(__funnelshift_r(w[0], w[1], 16), __funnelshift_r(w[1], w[2], 16),
+                                      __funnelshift_r(w[2], w[3], 16), __funnelshift_r(w[3], w[4], 16));
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  }
+};
+
+// out = in (+ add) for element-wide chunks: elements up to the first 16-byte boundary of `out` and behind the last one
+// singly, vectors in between.  A second output must lie like the first (the caller checks).
+template <typename T, bool ADD>
+__device__ __forceinline__ void og_move_unaligned(const char* in, const char* add, char* out0, char* out1, int n) {
+  constexpr int E = static_cast<int>(sizeof(T)), PER = 16 / E;
+  const char* out = out0 != nullptr ? out0 : out1;
+  const int head = min(n, static_cast<int>((16u - (static_cast<unsigned int>(reinterpret_cast<unsigned long long>(out)) & 15u)) & 15u) / E);
+  const int vecs = (n - head) / PER, tail = head + vecs * PER;
+  const int singles = head + (n - tail);                     // at most 2 * (PER - 1)
+  if (static_cast<int>(threadIdx.x) < singles) {
+    const int e = static_cast<int>(threadIdx.x) < head ? threadIdx.x : tail + threadIdx.x - head;
+    auto v = Access<E>::ld(in + static_cast<long long>(e) * E);
+    if (ADD) v = Wide<T, E>::add(v, Access<E>::ld(add + static_cast<long long>(e) * E));
+    if (out0 != nullptr) Access<E>::st(out0 + static_cast<long long>(e) * E, v);
+    if (out1 != nullptr) Access<E>::st(out1 + static_cast<long long>(e) * E, v);
+  }
+  const char* vin = in + head * E;
+  const char* vadd = ADD ? add + head * E : nullptr;
+  const unsigned int sh_in = static_cast<unsigned int>(reinterpret_cast<unsigned long long>(vin)) & 15u;
+  const unsigned int sh_add = ADD ? static_cast<unsigned int>(reinterpret_cast<unsigned long long>(vadd)) & 15u : 0u;
+  constexpr int U = ADD ? 2 : 4;
+#pragma unroll 1
+  for (int base = threadIdx.x; base < vecs; base += kOgData * U) {
+    Unaligned x[U], y[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long at = static_cast<long long>(min(base + u * kOgData, vecs - 1)) * 16;
+      x[u].load(vin + at);
+      if (ADD) y[u].load(vadd + at);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (base + u * kOgData < vecs) {
+        uint4 v = x[u].get(sh_in);
+        if (ADD) v = Wide<T, 16>::add(v, y[u].get(sh_add));
+        const long long at = head * E + static_cast<long long>(base + u * kOgData) * 16;
+        if (out0 != nullptr) *reinterpret_cast<uint4*>(out0 + at) = v;
+        if (out1 != nullptr) *reinterpret_cast<uint4*>(out1 + at) = v;
+      }
     }
   }
 }
@@ -261,7 +329,14 @@ template <typename T, int PROTO, int W>
 __device__ __forceinline__ void data_role(Shared& sh, const Waiter& w, unsigned long long limit) {
   for (unsigned int pass = 0;; ++pass) {
     const Job& job = sh.job[pass & 1];
-    if (!bar_wait(&sh.go[pass & 1], (pass >> 1) & 1u, limit)) return;
+    // the first warp waits for the job, the others for the first warp: a job may read what any warp wrote in the one
+    // before, and all warps leave together
+    if (threadIdx.x < 32) {
+      if (!bar_wait(&sh.go[pass & 1], (pass >> 1) & 1u, limit)) sh.leave = 1;
+      __syncwarp();
+    }
+    asm volatile("barrier.sync 1, %0;" ::"n"(kOgData) : "memory");
+    if (*reinterpret_cast<volatile int*>(&sh.leave) != 0) return;
     const int kind = job.kind;
     if (kind >= JOB_MOVE) {
       const int cnt = job.cnt, n = job.n;
@@ -273,8 +348,23 @@ __device__ __forceinline__ void data_role(Shared& sh, const Waiter& w, unsigned 
         if (kind == JOB_BATCH) {
           og_batch<T, W>(out0, job.src, j * job.src_step, job.nsrc, n);
         } else if (PROTO == PROTO_SIMPLE || kind == JOB_MOVE) {
-          if (add != nullptr) og_move<T, W, 4, true>(in, add, out0, out1, n);
-          else og_move<T, W, 8, false>(in, nullptr, out0, out1, n);
+          if constexpr (W == 16) {
+            if (add != nullptr) {
+              og_move<T, W, 4, true>(in, add, out0, out1, n);
+            } else {
+              og_move<T, W, 8, false>(in, nullptr, out0, out1, n);
+            }
+          } else {
+            const unsigned long long apart = reinterpret_cast<unsigned long long>(out0) ^ reinterpret_cast<unsigned long long>(out1);
+            if (out0 != nullptr && out1 != nullptr && (apart & 15ull) != 0) {
+              if (add != nullptr) og_move<T, W, 4, true>(in, add, out0, out1, n);
+              else og_move<T, W, 8, false>(in, nullptr, out0, out1, n);
+            } else if (add != nullptr) {
+              og_move_unaligned<T, true>(in, add, out0, out1, n);
+            } else {
+              og_move_unaligned<T, false>(in, nullptr, out0, out1, n);
+            }
+          }
         } else if constexpr (PROTO == PROTO_LL) {
           if (kind == JOB_SEND) og_move_ll<T, W, false, true>(in, nullptr, nullptr, out1, n, 0, job.flag_out, w, &sh.fail);
           else if (kind == JOB_RECV) og_move_ll<T, W, true, false>(in, add, out0, nullptr, n, job.flag_in, 0, w, &sh.fail);
@@ -292,11 +382,7 @@ __device__ __forceinline__ void data_role(Shared& sh, const Waiter& w, unsigned 
   }
 }
 
-struct Ends {                       // where this threadblock's flags live
-  unsigned long long *tail_out, *credit_out, *open_out, *progress_out;
-};
-
-__device__ __forceinline__ void signal_role(Shared& sh, const Ends& e, SyncPage* sync, int rank, int tb, int recv_peer, int chan,
+__device__ __forceinline__ void signal_role(Shared& sh, SyncPage* sync, int rank, int tb, int recv_peer, int chan,
                                             unsigned long long limit, unsigned long long* trace, int trace_steps) {
   for (unsigned int pass = 0;; ++pass) {
     const Job& job = sh.job[pass & 1];
@@ -310,11 +396,11 @@ __device__ __forceinline__ void signal_role(Shared& sh, const Ends& e, SyncPage*
       // one fence covers everything the step publishes; the credit alone needs none (the data warps have used what they
       // read from the FIFO slot before they came to the barrier)
       if (job.fence) fence_acq_rel_gpu();
-      if (job.tail != 0) st_relaxed_gpu(e.tail_out, job.tail);
-      if (job.opened != 0) st_relaxed_gpu(e.open_out, job.opened);
-      if (job.credit != 0) st_relaxed_gpu(e.credit_out, job.credit);
-      if (job.progress != 0) st_relaxed_gpu(e.progress_out, job.progress);
-      if (trace != nullptr) {
+      if (job.tail != 0) st_relaxed_gpu(job.tail_out, job.tail);
+      if (job.opened != 0) st_relaxed_gpu(job.open_out, job.opened);
+      if (job.credit != 0) st_relaxed_gpu(job.credit_out, job.credit);
+      if (job.progress != 0) st_relaxed_gpu(job.progress_out, job.progress);
+      if (trace != nullptr && job.traced) {
         const unsigned long long t2 = global_timer_ns();
         for (int s = job.step; s < job.step + job.steps && s < trace_steps; ++s) {
           unsigned long long* rec = trace + static_cast<long long>(s) * 6;
@@ -342,12 +428,13 @@ __device__ __forceinline__ int ld_signalled(const Shared& sh) {
 template <typename T, int PROTO, int W>
 __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(const __grid_constant__ OneGpuArgs a) {
   __shared__ Shared sh;
-  const int K = a.slices;
-  const int slice = static_cast<int>(blockIdx.x) % K;
-  const DevTb& tb = a.tbs[blockIdx.x / K];
+  const int K = a.ctas_per_tb, P = a.streams;
+  const int tb_index = static_cast<int>(blockIdx.x) / K, part = static_cast<int>(blockIdx.x) % K;
+  const DevTb& tb = a.tbs[tb_index];
   const int my_rank = tb.rank, my_tb = tb.tb_in_rank, nsteps = tb.nsteps;
-  const RankCtx& me = a.ranks[my_rank];
+  const OneGpuRank& me = a.ranks[my_rank];
   SyncPage* const sync = me.sync;
+  OneGpuFlags* const flags = me.flags;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const DevStep* sp = a.steps + tb.step_begin;
   if (nsteps <= kOgSmemSteps) {
@@ -359,6 +446,7 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
   if (threadIdx.x == 0) {
     sh.fail = 0;
     sh.signalled = 0;
+    sh.leave = 0;
     for (int i = 0; i < 2; ++i) {
       bar_init(&sh.go[i], 1);
       bar_init(&sh.done[i], kOgDataWarps);
@@ -370,36 +458,37 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
   w.deadline = global_timer_ns() + a.timeout_ns;
   const unsigned long long limit = w.deadline + 1000000000ull;
   const int send_peer = tb.send_peer, recv_peer = tb.recv_peer, chan = tb.chan;
-  const bool has_send = send_peer >= 0, has_recv = recv_peer >= 0;
-  // slice s of channel c uses the flags of channel c * K + s
-  const int vchan = chan * K + slice;
-  const int remote_idx = vchan * kMaxRanks + my_rank;
-  const int send_conn = vchan * kMaxRanks + send_peer, recv_conn = vchan * kMaxRanks + recv_peer;
-  Ends ends;
-  ends.tail_out = has_send ? &a.ranks[send_peer].sync->recv_tail[remote_idx] : nullptr;
-  ends.credit_out = has_recv ? &a.ranks[recv_peer].sync->send_head[remote_idx] : nullptr;
-  ends.open_out = has_recv ? &a.ranks[recv_peer].sync->recv_posted[remote_idx] : nullptr;
-  ends.progress_out = &sync->progress[my_tb * K + slice];
   __syncthreads();
 
   if (warp < kOgDataWarps) {
     data_role<T, PROTO, W>(sh, w, limit);
   } else if (warp == kOgDataWarps + 1) {
     if (lane == 0) {
-      unsigned long long* trace = (a.trace != nullptr && slice == 0) ? a.trace + static_cast<long long>(blockIdx.x / K) * a.trace_steps * 6 : nullptr;
-      signal_role(sh, ends, sync, my_rank, my_tb, recv_peer, chan, limit, trace, a.trace_steps);
+      unsigned long long* trace = (a.trace != nullptr && part == 0) ? a.trace + static_cast<long long>(tb_index) * a.trace_steps * 6 : nullptr;
+      signal_role(sh, sync, my_rank, my_tb, recv_peer, chan, limit, trace, a.trace_steps);
     }
   } else {
     // ------------------------------------------------------------------------------------------------ control warp
+    // P groups of 32 / P lanes; every lane of a group carries the state of the group's slice
+    const int LP = 32 / P, p = lane / LP, gl = lane % LP;
+    const unsigned int gmask = (LP == 32 ? ~0u : (1u << LP) - 1u) << (p * LP);
+    const bool has_send = send_peer >= 0, has_recv = recv_peer >= 0;
+    const int slices = K * P, slice = part * P + p;
+    const bool tracing = a.trace != nullptr && slice == 0;
+    // slice s of channel c uses the flags of channel c * slices + s, threadblock t the progress word t * slices + s
+    const int vchan = chan * slices + slice;
+    const int remote_idx = vchan * kMaxRanks + my_rank;
+    const int send_conn = vchan * kMaxRanks + send_peer, recv_conn = vchan * kMaxRanks + recv_peer;
     const long long C = a.chunk_elems;
     const long long lo = min(C, static_cast<long long>(slice) * a.slice_elems), hi = min(C, lo + a.slice_elems);
     const int iterations = static_cast<int>((hi - lo + a.tile_elems - 1) / a.tile_elems);
     const long long slot_bytes = a.slot_bytes;                  // of one slice
     char* const send_fifo = has_send ? a.ranks[send_peer].fifo + tb.send_fifo_off + slice * kFifoSlots * slot_bytes : nullptr;
     const char* const recv_fifo = has_recv ? me.fifo + tb.recv_fifo_off + slice * kFifoSlots * slot_bytes : nullptr;
-    unsigned long long sseq = has_send ? sync->send_seq[send_conn] : 0ull;
-    unsigned long long rseq = has_recv ? sync->recv_seq[recv_conn] : 0ull;
-    const unsigned long long sseq0 = sseq, rseq0 = rseq;
+    unsigned long long* const open_out = has_recv ? &a.ranks[recv_peer].flags->posted[remote_idx] : nullptr;
+    const unsigned long long sseq0 = has_send ? flags->send_seq[send_conn] : 0ull;
+    const unsigned long long rseq0 = has_recv ? flags->recv_seq[recv_conn] : 0ull;
+    unsigned long long sseq = sseq0, rseq = rseq0;
     // LL flags are unique per (launch, tile), as in exec_kernel.cu
     const unsigned int flag_epoch = static_cast<unsigned int>(epoch & 0xfffffull) << 12;
     const unsigned long long flag_epoch128 = epoch << 24;
@@ -408,38 +497,62 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
     unsigned long long opened = rseq0;
     unsigned long long head_seen = sseq0, posted_seen = 0;       // all credits of earlier launches have come back
     unsigned int mode_bits = 0;
-    unsigned int pass = 0;
-    bool stop = false;
     const long long esize = static_cast<long long>(sizeof(T));
+    unsigned int pass = 0;                                       // jobs handed over by this CTA
+    int last_pass = -1;                                          // the last one of this slice
+    int it = 0, s = 0;
+    bool finished = iterations == 0, setup = true, second = false;
+    // the step under way, filled in by the setup below
+    DevStep st;
+    int g = 0, nb = 1, V = 0, dep = 0;
+    long long tile_off = 0, fifo_chunk = 0;
+    const unsigned long long* flag = nullptr;
+    unsigned long long want = 0, word = 0, t0 = 0;
+    bool opens_here = false, can_direct_send = false, can_direct_recv = false;
+    unsigned int spins = 0;
 
-    for (int it = 0; it < iterations && !stop; ++it) {
-      const long long tile_off = lo + static_cast<long long>(it) * a.tile_elems;
-      const long long n = min(a.tile_elems, hi - tile_off);
-      const int V = static_cast<int>(n * esize / W);
-      const int lines = (2 * V + 14) / 15;
-      const long long fifo_chunk = PROTO == PROTO_SIMPLE ? static_cast<long long>(V) * W
-                                   : (PROTO == PROTO_LL ? static_cast<long long>(V) * LLPacket<W>::kBytes : static_cast<long long>(lines) * 128);
-      if (opening && tb.opens_at_start > 0) {
-        opened += tb.opens_at_start;
-        if (lane == 0) st_release_gpu(ends.open_out, opened);
+    // the next dependency of this lane at or behind `dep`
+    const auto next_dep = [&]() {
+      flag = nullptr;
+      for (; dep < g + nb; dep += LP - 3) {
+        const DevStep& sk = sp[s + dep];
+        if (sk.depid >= 0) {
+          flag = &flags->progress[sk.depid * slices + slice];
+          want = pack_progress(epoch, it, sk.deps + 1);
+          dep += LP - 3;
+          return;
+        }
       }
-      int s = 0;
-      while (s < nsteps && !stop) {
-        // nops that nobody waits for only add their dependency to the step behind them
-        int g = 0;
-        while (g < 8 && s + g + 1 < nsteps && sp[s + g].type == ST_NOP && sp[s + g].hasdep == 0) ++g;
-        const int ms = s + g;                                    // the step that moves something
-        const DevStep st = sp[ms];
-        const int nb = st.batch > 1 ? st.batch : 1;
-        const int last = ms + nb - 1;
-        const bool sends = is_send(st.type), recvs = is_recv(st.type);
-        const bool can_direct_send = PROTO == PROTO_SIMPLE && sends && (st.flags & SF_DIRECT_SEND) && ((a.direct_mask >> st.rbuf) & 1);
-        const bool can_direct_recv = PROTO == PROTO_SIMPLE && recvs && (st.flags & SF_DIRECT_RECV) && ((a.direct_mask >> st.dstbuf) & 1);
-        const bool always = (st.flags & SF_DIRECT_ALWAYS) != 0;
-        unsigned long long t0 = 0;
-        if (a.trace != nullptr && slice == 0) t0 = global_timer_ns();
+    };
 
-        // ---- bounds (as in exec_kernel.cu) ----
+    while (true) {
+      if (setup && !finished) {
+        // ---- the next step of this slice: sizes, bounds, and which flags its lanes look at ----
+        setup = false;
+        second = false;
+        if (s == 0) {
+          tile_off = lo + static_cast<long long>(it) * a.tile_elems;
+          V = static_cast<int>(min(a.tile_elems, hi - tile_off) * esize / W);
+          const int lines = (2 * V + 14) / 15;
+          fifo_chunk = PROTO == PROTO_SIMPLE ? static_cast<long long>(V) * W
+                       : (PROTO == PROTO_LL ? static_cast<long long>(V) * LLPacket<W>::kBytes : static_cast<long long>(lines) * 128);
+          if (opening && tb.opens_at_start > 0) {
+            opened += tb.opens_at_start;
+            if (gl == 0) st_release_gpu(open_out, opened);
+          }
+        }
+        // nops that nobody waits for only add their dependency to the step behind them
+        g = 0;
+        while (g < 8 && s + g + 1 < nsteps && sp[s + g].type == ST_NOP && sp[s + g].hasdep == 0) ++g;
+        st = sp[s + g];                                          // the step that moves something
+        nb = st.batch > 1 ? st.batch : 1;
+        const bool sends = is_send(st.type), recvs = is_recv(st.type);
+        can_direct_send = PROTO == PROTO_SIMPLE && sends && (st.flags & SF_DIRECT_SEND) && ((a.direct_mask >> st.rbuf) & 1);
+        can_direct_recv = PROTO == PROTO_SIMPLE && recvs && (st.flags & SF_DIRECT_RECV) && ((a.direct_mask >> st.dstbuf) & 1);
+        opens_here = opening && st.opens_before > 0;
+        if (tracing) t0 = global_timer_ns();
+
+        // bounds, as in exec_kernel.cu
         bool in_bounds = true;
         long long worst = 0;
         if (st.type != ST_NOP) {
@@ -449,181 +562,202 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
           if (uses_dst && (static_cast<long long>(st.dstoff) + st.cnt) * C > me.buf_elems[st.dstbuf]) { in_bounds = false; worst = st.dstoff; }
           if (can_direct_send && (static_cast<long long>(st.roff) + st.cnt) * C > a.ranks[send_peer].buf_elems[st.rbuf]) { in_bounds = false; worst = st.roff; }
           if ((sends || recvs) && st.cnt * fifo_chunk > slot_bytes) { in_bounds = false; worst = -1; }
-        }
-        if (nb > 1) {                                            // one batch member per lane
-          bool ok = true;
-          long long off = 0;
-          if (lane >= 1 && lane < nb) {
-            const DevStep sk = sp[ms + lane];
-            if (sk.type == ST_RE && (static_cast<long long>(sk.srcoff) + sk.cnt) * C > me.buf_elems[sk.srcbuf]) { ok = false; off = sk.srcoff; }
+          for (int k = 1; k < nb; ++k) {
+            const DevStep& sk = sp[s + g + k];
+            if (sk.type == ST_RE && (static_cast<long long>(sk.srcoff) + sk.cnt) * C > me.buf_elems[sk.srcbuf]) { in_bounds = false; worst = sk.srcoff; }
           }
-          const unsigned int bad = __ballot_sync(kFullWarp, !ok);
-          if (bad != 0 && in_bounds) { in_bounds = false; worst = __shfl_sync(kFullWarp, off, __ffs(bad) - 1); }
+        }
+        if (!in_bounds) {
+          if (gl == 0) record_failure(sync, STATUS_BOUNDS, my_rank, my_tb, s + g, it, st.type, static_cast<unsigned int>(worst));
+          *reinterpret_cast<volatile int*>(&sh.fail) = 1;
         }
 
-        // ---- waits: one flag per lane ----
-        // lane 0: a free FIFO slot; lane 1: the tile; lane 2: may this tile go straight into the receiver's slot?;
-        // lanes 3..: the dependencies of the pass.  A receive that opens its own slot does so after the dependencies,
-        // so it polls the tile in a second round.
+        // lane 0 of the group: a free FIFO slot; 1: the tile; 2: may the tile go straight into the receiver's slot? (looked
+        // at once); 3..: the dependencies.  A receive that opens its own slot looks for the tile afterwards.
         const unsigned long long want_head = sseq + 1 > kFifoSlots ? sseq + 1 - kFifoSlots : 0;
-        const bool opens_here = opening && st.opens_before > 0;
-        unsigned int failed_lane = 0;
-        unsigned long long word = 0;
-        const unsigned long long* flag = nullptr;
-        unsigned long long want = 0, mask = ~0ull;
-        if (lane == 0 && sends && head_seen < want_head) { flag = &sync->send_head[send_conn]; want = want_head; }
-        if (lane == 1 && recvs && PROTO == PROTO_SIMPLE && !opens_here) { flag = &sync->recv_tail[recv_conn]; want = rseq + 1; mask = kTailCountMask; }
-        if (lane == 2 && can_direct_send && !always && posted_seen < sseq + 1) flag = &sync->recv_posted[send_conn];   // looked at once
-        if (lane >= 3 && lane < 3 + g + nb && in_bounds) {
-          const DevStep& sk = sp[s + lane - 3];
-          if (sk.depid >= 0) { flag = &sync->progress[sk.depid * K + slice]; want = pack_progress(epoch, it, sk.deps + 1); }
+        flag = nullptr;
+        want = 0;
+        word = 0;
+        if (gl == 0) {
+          if (sends && head_seen < want_head) { flag = &flags->head[send_conn]; want = want_head; }
+        } else if (gl == 1) {
+          if (recvs && PROTO == PROTO_SIMPLE && !opens_here) { flag = &flags->tail[recv_conn]; want = rseq + 1; }
+        } else if (gl == 2) {
+          if (can_direct_send && (st.flags & SF_DIRECT_ALWAYS) == 0 && posted_seen < sseq + 1) flag = &flags->posted[send_conn];
+        } else {
+          dep = gl - 3;
+          next_dep();
         }
-        if (!in_bounds) flag = nullptr;
-        // the job slot of two passes ago must have been read by the signal warp before it is written below
-        const int need_sig = static_cast<int>(pass) - 1;
-#pragma unroll 1
-        for (int round = 0; round < (opens_here ? 2 : 1) && failed_lane == 0 && in_bounds; ++round) {
-          if (round == 1) {
-            // the slot may be opened: what came before this step has been signalled, its dependencies have arrived
-            for (unsigned int i = 1; ld_signalled(sh) < static_cast<int>(pass) && failed_lane == 0; ++i)
-              if ((i & 255u) == 0 && (*reinterpret_cast<volatile int*>(&sh.fail) != 0 || w.expired())) failed_lane = 32;
-            failed_lane = __reduce_max_sync(kFullWarp, failed_lane);
-            opened += st.opens_before;
-            if (lane == 0) st_release_gpu(ends.open_out, opened);
-            flag = nullptr;
-            if (lane == 1 && recvs) { flag = &sync->recv_tail[recv_conn]; want = rseq + 1; mask = kTailCountMask; }
-          }
-          bool pending = flag != nullptr;
-          unsigned int spins = 0;
-          while (__any_sync(kFullWarp, pending)) {
-            if (pending) {
-              word = ld_acquire_gpu(flag);
-              if ((word & mask) >= want) pending = false;
-            }
-            if ((++spins & 127u) == 0) {
-              const bool give_up = lane == 0 && (*reinterpret_cast<volatile int*>(&sh.fail) != 0 || w.expired());
-              if (__any_sync(kFullWarp, give_up)) {
-                const unsigned int open_lanes = __ballot_sync(kFullWarp, pending);
-                if (open_lanes != 0) failed_lane = static_cast<unsigned int>(__ffs(open_lanes));
-                break;
-              }
-            }
-          }
-        }
-        __syncwarp();
-        for (unsigned int i = 1; ld_signalled(sh) < need_sig && failed_lane == 0; ++i)
-          if ((i & 255u) == 0 && w.expired()) failed_lane = 32;
-        failed_lane = __reduce_max_sync(kFullWarp, failed_lane);
-        if (sends) head_seen = max(head_seen, __shfl_sync(kFullWarp, word, 0));
-        if (can_direct_send && !always && posted_seen < sseq + 1) posted_seen = __shfl_sync(kFullWarp, word, 2);
-        const bool direct_send = can_direct_send && (always || posted_seen >= sseq + 1);
-        const unsigned long long tail_word = __shfl_sync(kFullWarp, word, 1);
-        const bool direct_recv = can_direct_recv && ((tail_word >> (kTailModeShift + static_cast<int>(rseq % kFifoSlots))) & 1ull) != 0;
+      }
 
-        if (!in_bounds || failed_lane != 0 || *reinterpret_cast<volatile int*>(&sh.fail) != 0) {
-          // a flag-in-data poll that ran out of time is recorded by the signal warp, which knows its step
-          if (lane == 0 && *reinterpret_cast<volatile int*>(&sh.fail) == 0) {
+      // ---- one look at every flag ----
+      if (flag != nullptr) {
+        word = ld_acquire_gpu(flag);
+        if ((gl == 1 ? word & kTailCountMask : word) >= want) {
+          flag = nullptr;
+          if (gl >= 3) next_dep();
+        }
+      }
+      __syncwarp();
+      const int signalled = __shfl_sync(kFullWarp, ld_signalled(sh), 0);
+      const unsigned int waiting = __ballot_sync(kFullWarp, flag != nullptr);
+      bool ready = !finished && (waiting & gmask) == 0;
+      if (ready && opens_here && !second) {
+        // the slot may be opened once this slice's last job has been signalled (its dependencies have arrived)
+        if (signalled > last_pass) {
+          opened += st.opens_before;
+          if (gl == 0) st_release_gpu(open_out, opened);
+          if (gl == 1) { flag = &flags->tail[recv_conn]; want = rseq + 1; }
+          second = true;
+        }
+        ready = false;
+      }
+      unsigned int ready_set = __ballot_sync(kFullWarp, ready && gl == 0);
+      const bool failed = __any_sync(kFullWarp, *reinterpret_cast<volatile int*>(&sh.fail) != 0);
+      if (failed) break;                                         // recorded by whoever raised it
+      if (ready_set == 0) {
+        if (__all_sync(kFullWarp, finished)) break;
+        if ((++spins & 127u) == 0 && __any_sync(kFullWarp, lane == 0 && w.expired())) {
+          const unsigned int open_lanes = __ballot_sync(kFullWarp, flag != nullptr);
+          const int who = open_lanes != 0 ? __ffs(open_lanes) - 1 : 0;
+          if (lane == who) {
             unsigned int code = STATUS_ABORTED, aux0 = 0, aux1 = 0;
-            if (!in_bounds) { code = STATUS_BOUNDS; aux0 = st.type; aux1 = static_cast<unsigned int>(worst); }
-            else if (failed_lane == 1) { code = STATUS_TIMEOUT_CREDIT; aux0 = send_peer; aux1 = chan; }
-            else if (failed_lane == 2) { code = STATUS_TIMEOUT_DATA; aux0 = recv_peer; aux1 = chan; }
-            else if (failed_lane > 3 && failed_lane < 32) { code = STATUS_TIMEOUT_DEP; aux0 = sp[s + failed_lane - 4].depid; aux1 = sp[s + failed_lane - 4].deps; }
-            record_failure(sync, code, my_rank, my_tb, ms, it, aux0, aux1);
+            if (open_lanes != 0) {
+              if (gl == 0) { code = STATUS_TIMEOUT_CREDIT; aux0 = send_peer; aux1 = chan; }
+              else if (gl == 1) { code = STATUS_TIMEOUT_DATA; aux0 = recv_peer; aux1 = chan; }
+              else if (gl >= 3) { const DevStep& sk = sp[s + dep - (LP - 3)]; code = STATUS_TIMEOUT_DEP; aux0 = sk.depid; aux1 = sk.deps; }
+            }
+            record_failure(sync, code, my_rank, my_tb, s + g, it, aux0, aux1);
             *reinterpret_cast<volatile int*>(&sh.fail) = 1;
           }
-          stop = true;
+          __syncwarp();
           break;
         }
+        continue;
+      }
 
-        // ---- the job ----
-        if (lane == 0) {
-          Job& job = sh.job[pass & 1];
-          char* const sbase = static_cast<char*>(me.buf[st.srcbuf]) + (static_cast<long long>(st.srcoff) * C + tile_off) * esize;
-          char* const dbase = static_cast<char*>(me.buf[st.dstbuf]) + (static_cast<long long>(st.dstoff) * C + tile_off) * esize;
-          const char* fifo_in = recvs ? recv_fifo + (rseq % kFifoSlots) * slot_bytes : nullptr;
-          char* out1 = nullptr;
-          if (sends)
-            out1 = direct_send ? static_cast<char*>(a.ranks[send_peer].buf[st.rbuf]) + (static_cast<long long>(st.roff) * C + tile_off) * esize
-                               : send_fifo + (sseq % kFifoSlots) * slot_bytes;
-          const long long chunk_step = C * esize;
-          int kind = JOB_MOVE;
-          const char *in = nullptr, *add = nullptr;
-          char* out0 = nullptr;
-          long long in_step = chunk_step;
-          if (recvs && !direct_recv) { in = fifo_in; in_step = fifo_chunk; }
-          switch (st.type) {
-            case ST_SEND: in = sbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_SEND; break;
-            case ST_RECV:
-              out0 = dbase;
-              kind = PROTO == PROTO_SIMPLE ? (direct_recv ? JOB_NONE : JOB_MOVE) : JOB_RECV;
-              break;
-            case ST_RCS:
-              if (direct_recv) in = dbase; else out0 = dbase;
-              kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_BOTH;
-              break;
-            case ST_RRC: add = dbase; out0 = dbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_RECV; break;
-            case ST_RRS: add = dbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_BOTH; break;
-            case ST_RRCS: add = dbase; out0 = dbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_BOTH; break;
-            case ST_CPY: in = sbase; out0 = dbase; break;
-            case ST_RE:
-              if (nb == 1) { in = dbase; add = sbase; out0 = dbase; }
-              else { in = dbase; out0 = dbase; kind = JOB_BATCH; }
-              break;
-            default: kind = JOB_NONE; break;
-          }
-          int nsrc = 0;
-          unsigned int more = opening ? st.opens_after : 0;
-          bool any_dep = st.hasdep != 0;
-          for (int k = 0; k < nb; ++k) {
-            const DevStep& sk = sp[ms + k];
-            if (k > 0) {
-              if (opening) more += sk.opens_after;
-              any_dep = any_dep || sk.hasdep != 0;
-            }
-            if (kind == JOB_BATCH && sk.type == ST_RE && nsrc < kMaxBatch)
-              job.src[nsrc++] = static_cast<char*>(me.buf[sk.srcbuf]) + (static_cast<long long>(sk.srcoff) * C + tile_off) * esize;
-          }
-          job.in = in; job.add = add; job.out0 = out0; job.out1 = out1;
-          job.in_step = in_step; job.add_step = chunk_step; job.out0_step = chunk_step;
-          job.out1_step = direct_send ? chunk_step : fifo_chunk;
-          job.src_step = chunk_step;
-          job.kind = kind; job.cnt = st.cnt; job.n = V; job.nsrc = nsrc;
-          job.flag_in = flag_epoch | (static_cast<unsigned int>((rseq - rseq0) % 4095ull) + 1u);
-          job.flag_out = flag_epoch | (static_cast<unsigned int>((sseq - sseq0) % 4095ull) + 1u);
-          job.flag_in128 = flag_epoch128 | (rseq - rseq0 + 1);
-          job.flag_out128 = flag_epoch128 | (sseq - sseq0 + 1);
+      // ---- hand the jobs that are ready over, one after the other ----
+      bool stuck = false;
+      while (ready_set != 0) {
+        const int q = __ffs(ready_set) - 1;                      // first lane of the group
+        ready_set &= ready_set - 1;
+        // the job slot of two passes ago must have been read by the signal warp
+        for (unsigned int i = 1; ld_signalled(sh) < static_cast<int>(pass) - 1; ++i)
+          if ((i & 255u) == 0 && global_timer_ns() > limit) { stuck = true; break; }
+        stuck = __any_sync(kFullWarp, stuck);
+        if (stuck) break;
+        const unsigned long long w_head = __shfl_sync(kFullWarp, word, q), w_tail = __shfl_sync(kFullWarp, word, q + 1),
+                                 w_posted = __shfl_sync(kFullWarp, word, q + 2);
+        if (p == q / LP) {
+          const bool sends = is_send(st.type), recvs = is_recv(st.type), always = (st.flags & SF_DIRECT_ALWAYS) != 0;
+          const int last = s + g + nb - 1;
+          if (sends) head_seen = max(head_seen, w_head);
+          if (can_direct_send && !always) posted_seen = max(posted_seen, w_posted);
+          const bool direct_send = can_direct_send && (always || posted_seen >= sseq + 1);
+          const bool direct_recv = can_direct_recv && ((w_tail >> (kTailModeShift + static_cast<int>(rseq % kFifoSlots))) & 1ull) != 0;
           const bool publishes_tile = sends && PROTO == PROTO_SIMPLE;
           if (publishes_tile) {
             const unsigned int bit = 1u << static_cast<int>(sseq % kFifoSlots);
             mode_bits = direct_send ? (mode_bits | bit) : (mode_bits & ~bit);
           }
-          job.tail = publishes_tile ? (static_cast<unsigned long long>(mode_bits) << kTailModeShift) | (sseq + 1) : 0ull;
-          job.opened = more > 0 ? opened + more : 0ull;
-          job.credit = recvs ? rseq + 1 : 0ull;
-          job.progress = any_dep ? pack_progress(epoch, it, last + 1) : 0ull;
-          job.fence = publishes_tile || more > 0 || any_dep;
+          unsigned int more = opening ? st.opens_after : 0;
+          bool any_dep = st.hasdep != 0;
+          for (int k = 1; k < nb; ++k) {
+            const DevStep& sk = sp[s + g + k];
+            if (opening) more += sk.opens_after;
+            any_dep = any_dep || sk.hasdep != 0;
+          }
           opened += more;
-          job.step = s; job.steps = g + nb; job.iter = it;
-          if (a.trace != nullptr && slice == 0) { job.t0 = t0; job.t1 = global_timer_ns(); }
-          bar_arrive(&sh.go[pass & 1]);
+          if (gl == 0) {
+            Job& job = sh.job[pass & 1];
+            const long long chunk_step = C * esize;
+            char* const sbase = static_cast<char*>(me.buf[st.srcbuf]) + (static_cast<long long>(st.srcoff) * C + tile_off) * esize;
+            char* const dbase = static_cast<char*>(me.buf[st.dstbuf]) + (static_cast<long long>(st.dstoff) * C + tile_off) * esize;
+            char* out1 = nullptr;
+            if (sends)
+              out1 = direct_send ? static_cast<char*>(a.ranks[send_peer].buf[st.rbuf]) + (static_cast<long long>(st.roff) * C + tile_off) * esize
+                                 : send_fifo + (sseq % kFifoSlots) * slot_bytes;
+            int kind = JOB_MOVE;
+            const char *in = nullptr, *add = nullptr;
+            char* out0 = nullptr;
+            long long in_step = chunk_step;
+            if (recvs && !direct_recv) { in = recv_fifo + (rseq % kFifoSlots) * slot_bytes; in_step = fifo_chunk; }
+            switch (st.type) {
+              case ST_SEND: in = sbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_SEND; break;
+              case ST_RECV:
+                out0 = dbase;
+                kind = PROTO == PROTO_SIMPLE ? (direct_recv ? JOB_NONE : JOB_MOVE) : JOB_RECV;
+                break;
+              case ST_RCS:
+                if (direct_recv) in = dbase; else out0 = dbase;
+                kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_BOTH;
+                break;
+              case ST_RRC: add = dbase; out0 = dbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_RECV; break;
+              case ST_RRS: add = dbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_BOTH; break;
+              case ST_RRCS: add = dbase; out0 = dbase; kind = PROTO == PROTO_SIMPLE ? JOB_MOVE : JOB_BOTH; break;
+              case ST_CPY: in = sbase; out0 = dbase; break;
+              case ST_RE:
+                in = dbase; out0 = dbase;
+                if (nb == 1) add = sbase; else kind = JOB_BATCH;
+                break;
+              default: kind = JOB_NONE; break;
+            }
+            int nsrc = 0;
+            if (kind == JOB_BATCH) {
+              for (int k = 0; k < nb; ++k) {
+                const DevStep& sk = sp[s + g + k];
+                if (sk.type == ST_RE && nsrc < kMaxBatch)
+                  job.src[nsrc++] = static_cast<char*>(me.buf[sk.srcbuf]) + (static_cast<long long>(sk.srcoff) * C + tile_off) * esize;
+              }
+            }
+            job.in = in; job.add = add; job.out0 = out0; job.out1 = out1;
+            job.in_step = in_step; job.add_step = chunk_step; job.out0_step = chunk_step;
+            job.out1_step = direct_send ? chunk_step : fifo_chunk;
+            job.src_step = chunk_step;
+            job.kind = kind; job.cnt = st.cnt; job.n = V; job.nsrc = nsrc;
+            if (PROTO != PROTO_SIMPLE) {
+              job.flag_in = flag_epoch | (static_cast<unsigned int>((rseq - rseq0) % 4095ull) + 1u);
+              job.flag_out = flag_epoch | (static_cast<unsigned int>((sseq - sseq0) % 4095ull) + 1u);
+              job.flag_in128 = flag_epoch128 | (rseq - rseq0 + 1);
+              job.flag_out128 = flag_epoch128 | (sseq - sseq0 + 1);
+            }
+            job.tail = publishes_tile ? (static_cast<unsigned long long>(mode_bits) << kTailModeShift) | (sseq + 1) : 0ull;
+            job.opened = more > 0 ? opened : 0ull;
+            job.credit = recvs ? rseq + 1 : 0ull;
+            job.progress = any_dep ? pack_progress(epoch, it, last + 1) : 0ull;
+            job.tail_out = has_send ? &a.ranks[send_peer].flags->tail[remote_idx] : nullptr;
+            job.credit_out = has_recv ? &a.ranks[recv_peer].flags->head[remote_idx] : nullptr;
+            job.open_out = open_out;
+            job.progress_out = &flags->progress[my_tb * slices + slice];
+            job.fence = publishes_tile || more > 0 || any_dep;
+            job.step = s; job.steps = g + nb; job.iter = it; job.traced = tracing;
+            if (tracing) { job.t0 = t0; job.t1 = global_timer_ns(); }
+            bar_arrive(&sh.go[pass & 1]);
+          }
+          if (sends) ++sseq;
+          if (recvs) ++rseq;
+          last_pass = static_cast<int>(pass);
+          s = last + 1;
+          if (s >= nsteps) { s = 0; finished = ++it >= iterations; }
+          setup = true;
         }
-        if (opening) opened = __shfl_sync(kFullWarp, opened, 0);
         ++pass;
-        if (sends) ++sseq;
-        if (recvs) ++rseq;
-        s = last + 1;
+        spins = 0;
+        __syncwarp();
       }
+      if (stuck) break;
     }
     // the last pass: tells data and signal warps to leave
-    const int need_sig = static_cast<int>(pass) - 1;
-    for (unsigned int i = 1; ld_signalled(sh) < need_sig; ++i)
+    for (unsigned int i = 1; ld_signalled(sh) < static_cast<int>(pass) - 1; ++i)
       if ((i & 255u) == 0 && global_timer_ns() > limit) break;
     __syncwarp();
     if (lane == 0) {
       sh.job[pass & 1].kind = JOB_EXIT;
       bar_arrive(&sh.go[pass & 1]);
-      if (has_send) sync->send_seq[send_conn] = sseq;
-      if (has_recv) sync->recv_seq[recv_conn] = rseq;
+    }
+    if (gl == 0) {
+      if (has_send) flags->send_seq[send_conn] = sseq;
+      if (has_recv) flags->recv_seq[recv_conn] = rseq;
     }
   }
   // every role of this CTA has left: the last CTA of the rank advances its launch epoch
@@ -666,13 +800,13 @@ const void* pick_kernel(int dtype, int proto, int width) {
 
 }  // namespace
 
-// `slices` CTAs per threadblock; always cooperative unless the caller vouches for an otherwise idle GPU.
+// `args.ctas_per_tb` CTAs per threadblock; cooperative unless the caller vouches for an otherwise idle GPU.
 cudaError_t launch_exec_one_gpu(const OneGpuArgs& args, int dtype, int proto, int width, int tbs, cudaStream_t stream, bool cooperative) {
   const void* fn = pick_kernel(dtype, proto, width);
   if (fn == nullptr) return cudaErrorInvalidValue;
   OneGpuArgs copy = args;
   void* params[] = {&copy};
-  const dim3 grid(static_cast<unsigned int>(tbs * args.slices)), block(kOgThreads);
+  const dim3 grid(static_cast<unsigned int>(tbs * args.ctas_per_tb)), block(kOgThreads);
   if (cooperative) return cudaLaunchCooperativeKernel(fn, grid, block, params, 0, stream);
   return cudaLaunchKernel(fn, grid, block, params, 0, stream);
 }

@@ -142,20 +142,37 @@ struct ExecArgs {
   int trace_steps;            // steps per threadblock the trace has room for
 };
 
-// Launch of the one-GPU interpreter (exec_one_gpu.cu): every rank on this device, each threadblock run by `slices` CTAs.
+// The one-GPU interpreter (exec_one_gpu.cu): every rank on this device, each threadblock run by `ctas_per_tb` CTAs with
+// `streams` slices of every chunk each.  Its flags are those of SyncPage, one set per (connection, slice).
+constexpr int kOneGpuChannels = 1024;                  // channels x slices
+constexpr int kOneGpuConns = kOneGpuChannels * kMaxRanks;
+constexpr int kOneGpuProgress = 4096;                  // threadblocks of a rank x slices
+struct alignas(128) OneGpuFlags {
+  unsigned long long tail[kOneGpuConns], head[kOneGpuConns], posted[kOneGpuConns];
+  unsigned long long send_seq[kOneGpuConns], recv_seq[kOneGpuConns];
+  unsigned long long progress[kOneGpuProgress];
+};
+struct OneGpuRank {
+  SyncPage* sync;             // launch epoch and status words
+  OneGpuFlags* flags;
+  char* fifo;
+  void* buf[3];
+  long long buf_elems[3];
+};
 struct OneGpuArgs {
   const DevTb* tbs;
   const DevStep* steps;
   long long chunk_elems;      // elements per chunk
-  long long slice_elems;      // elements of each chunk that one CTA of a threadblock works on (the last may have fewer)
+  long long slice_elems;      // elements of each chunk in one slice (the last may have fewer)
   long long tile_elems;       // elements of a slice processed per iteration
   long long slot_bytes;       // FIFO slot of one slice
   unsigned long long timeout_ns;
   unsigned long long* trace;  // as in ExecArgs; slice 0 of every threadblock records
   int trace_steps;
-  int slices;
+  int ctas_per_tb;
+  int streams;                // slices per CTA: 1, 2 or 4 (more than one only under the Simple protocol)
   int direct_mask;
-  RankCtx ranks[kMaxRanks];
+  OneGpuRank ranks[kMaxRanks];
 };
 
 static_assert(sizeof(DevStep) == 32 && sizeof(DevTb) == 64, "layout shared with msccl/runtime/plan.py");

@@ -27,6 +27,7 @@ from msccl.runtime.native import load
 
 SYNC_BYTES = 128 * 1024
 _RANKCTX = struct.Struct('<2Q3Q3q')
+_ONE_GPU_RANK = '3Q3Q3q'            # OneGpuRank of csrc/msccl_device.h: addresses, buffers, their sizes
 
 
 def _align(v, a):
@@ -59,11 +60,12 @@ class Communicator:
         self.timeout_ns = int(float(os.environ.get('MSCCL_TIMEOUT_S', '20')) * 1e9)
 
     # ------------------------------------------------------------------ layout
-    def _set_layout(self, world, ll_max_bytes, fifo_bytes, arena_bytes):
+    def _set_layout(self, world, ll_max_bytes, fifo_bytes, arena_bytes, flag_bytes=0):
         self.ll_slot_bytes = _align(2 * ll_max_bytes, 1024)
         self.off_fused = SYNC_BYTES
         self.off_staging = 2 * SYNC_BYTES
-        self.off_fifo = _align(self.off_staging + 2 * world * self.ll_slot_bytes, 1 << 16)
+        self.off_flags = _align(self.off_staging + 2 * world * self.ll_slot_bytes, 1 << 16)     # one-GPU interpreter
+        self.off_fifo = _align(self.off_flags + flag_bytes, 1 << 16)
         self.fifo_bytes = fifo_bytes
         self.off_arena = _align(self.off_fifo + fifo_bytes, 1 << 21)
         self.arena_bytes = arena_bytes
@@ -99,7 +101,8 @@ class Communicator:
         self.emulated_mode = True
         self.device = torch.cuda.current_device() if device is None else device
         torch.cuda.set_device(self.device)
-        self._set_layout(world, ll_max_bytes, fifo_bytes, arena_bytes)
+        self._set_layout(world, ll_max_bytes, fifo_bytes, arena_bytes, self.native.layout()['sizeof_OneGpuFlags'])
+        self.one_gpu_table = struct.Struct('<' + _ONE_GPU_RANK * world)
         for _ in range(world):
             ptr = self.native.device_malloc(self.heap_bytes, False)
             self.native.device_memset(ptr, 0, self.off_arena)      # flags and FIFOs (packets carry their flags)
@@ -266,6 +269,11 @@ class Communicator:
             n = sizes.get(r, (0, 0, 0))
             out.append(_RANKCTX.pack(self.sync_ptr(r), self.fifo_ptr(r), b[0], b[1], b[2], n[0], n[1], n[2]))
         return b''.join(out)
+
+    def one_gpu_addresses(self, r):
+        """What stands in front of the buffers in rank ``r``'s entry of the one-GPU interpreter's rank table."""
+        base = self.heap_ptrs[r]
+        return base, base + self.off_flags, base + self.off_fifo
 
     # -------------------------------------------------------- symmetric tensors
     def symmetric_empty(self, numel, dtype):

@@ -60,7 +60,9 @@ class DevicePlan:
         # with every rank on this GPU a hop between threadblocks costs more than the add it passes on
         self.host: HostPlan = compile_plan(fold_reduce_chains(algo) if comm.emulated_mode else algo, comm.local_ranks,
                                            self.slot_bytes)
-        self.geometry = {}         # emulated mode: (chunk elements, element size, width, proto) -> launch geometry
+        self.geometry = {}         # emulated mode: (chunk elements, dtype, width, direct) -> launch geometry
+        self.rank_info = [(self.host.extents[r]['i'], self.host.extents[r]['o'], self.host.extents[r]['s'], algo.gpus[r].o_chunks,
+                           comm.one_gpu_addresses(r)) for r in comm.local_ranks] if comm.emulated_mode else []
         nat = comm.native
         self.dev_tbs = nat.upload(self.host.tb_bytes)
         self.dev_steps = nat.upload(self.host.step_bytes)
@@ -139,6 +141,8 @@ class Executor:
         outputs = outputs or {}
         if plan.nvls_kind is not None:
             return self._run_in_switch(plan, inputs, outputs, stream)
+        if comm.emulated_mode and not trace and declared_elems is None and not (algo.inplace and algo.coll == 'allgather'):
+            return self._run_one_gpu(plan, inputs, outputs, stream, direct)
         first = inputs[comm.local_ranks[0]]
         dtype = first.dtype
         if dtype not in DTYPE_CODES:
@@ -202,12 +206,7 @@ class Executor:
             tile, iterations = tile_geometry(plan.host, chunk, esize, plan.slot_bytes, width, proto)
         stream_h = (stream or torch.cuda.current_stream()).cuda_stream
         nat = comm.native
-        key = (DTYPE_CODES[dtype], proto, width)
-        if key not in self._checked_grid:
-            self._checked_grid[key] = (nat.max_coresident_one_gpu if comm.emulated_mode else nat.max_coresident_ctas)(*key)
-        if plan.grid > self._checked_grid[key]:
-            raise PlanError(f'{plan.grid} threadblocks cannot be co-resident on this device '
-                            f'(limit {self._checked_grid[key]})')
+        key = self._check_grid(plan, dtype, proto, width)
         trace_ptr, trace_steps = 0, 0
         if trace:
             trace_steps = max(1, max(len(tb.steps) for g in plan.host.algo.gpus for tb in g.tbs))
@@ -215,15 +214,12 @@ class Executor:
             self._trace_shape = (plan, trace_steps)
             trace_ptr = self._trace.data_ptr()
         if comm.emulated_mode:
-            geometry = plan.geometry.get((chunk, esize, width, proto))
-            if geometry is None:
-                geometry = plan.geometry[(chunk, esize, width, proto)] = one_gpu_geometry(
-                    plan.host, chunk, esize, plan.slot_bytes, width, proto, self._checked_grid[key])
-            slices, slice_elems, tile, slot = geometry
+            geometry = self._one_gpu_geometry(plan, chunk, dtype, esize, width, proto, direct)
             self.last_direct_mask = 7 if direct else 0
-            nat.launch_one_gpu(plan.dev_tbs, plan.dev_steps, comm.rankctx_bytes(buffers, sizes), chunk, slice_elems, tile, slot,
-                               slices, plan.grid, key[0], proto, width, comm.timeout_ns, self.last_direct_mask, stream_h,
-                               self.cooperative, trace_ptr, trace_steps)
+            words = [w for r in comm.local_ranks for w in (*comm.one_gpu_addresses(r), *buffers[r], *sizes[r])]
+            nat.launch_one_gpu(plan.dev_tbs, plan.dev_steps, comm.one_gpu_table.pack(*words), chunk, geometry, plan.grid, key[0],
+                               proto, width, comm.timeout_ns, self.last_direct_mask, stream_h, self.cooperative, trace_ptr,
+                               trace_steps)
         else:
             r = comm.rank
             sym_off, mask = [-1, -1, -1], 0
@@ -237,6 +233,79 @@ class Executor:
             nat.launch(plan.dev_tbs, plan.dev_steps, comm.dev_rankctx, geom, comm.timeout_ns, stream_h, self.cooperative,
                        bufs=list(buffers[r]), elems=list(sizes[r]), peer_heaps=list(comm.heap_ptrs), sym_off=sym_off,
                        direct_mask=mask, trace=trace_ptr, trace_steps=trace_steps, wait_mode=self.wait_mode)
+        self.launches += 1
+        return results
+
+    def _check_grid(self, plan, dtype, proto, width):
+        key = (DTYPE_CODES[dtype], proto, width)
+        if key not in self._checked_grid:
+            nat = self.comm.native
+            self._checked_grid[key] = (nat.max_coresident_one_gpu if self.comm.emulated_mode else nat.max_coresident_ctas)(*key)
+        if plan.grid > self._checked_grid[key]:
+            raise PlanError(f'{plan.grid} threadblocks cannot be co-resident on this device '
+                            f'(limit {self._checked_grid[key]})')
+        return key
+
+    def _one_gpu_geometry(self, plan, chunk, dtype, esize, width, proto, direct):
+        key = (chunk, dtype, width, bool(direct))
+        geometry = plan.geometry.get(key)
+        if geometry is None:
+            most = self._checked_grid[self._check_grid(plan, dtype, proto, width)]
+            if len(plan.geometry) >= 1024:
+                plan.geometry.clear()
+            geometry = plan.geometry[key] = one_gpu_geometry(plan.host, chunk, esize, plan.slot_bytes, width, proto, most, bool(direct))
+        return geometry
+
+    def _run_one_gpu(self, plan, inputs, outputs, stream, direct):
+        """``run`` for a communicator with every rank on this GPU: the same checks in one pass over the ranks, written for
+        calls whose kernel takes a few microseconds (8 ranks: 33 us of host time before, about 15 this way)."""
+        comm = self.comm
+        first = inputs[0]
+        dtype = first.dtype
+        if dtype not in DTYPE_CODES:
+            raise PlanError(f'unsupported dtype {dtype}')
+        esize = first.element_size()
+        chunk = chunk_geometry(plan.algo, 0, first.numel())
+        if direct == 'auto':
+            direct = os.environ.get('MSCCL_DIRECT', '1') != '0'
+        words, results, bits = [], {}, 0
+        for r, (read, written, scratch_chunks, out_chunks, addresses) in enumerate(plan.rank_info):
+            t_in = inputs[r]
+            assert t_in.is_cuda and t_in.is_contiguous() and t_in.dtype == dtype
+            in_ptr, in_elems = t_in.data_ptr(), t_in.numel()
+            if in_elems < read * chunk:
+                raise PlanError(f'rank {r}: input of {in_elems} elements, program reads {read * chunk}')
+            out_ptr = out_elems = scratch_ptr = scratch_elems = 0
+            if written:
+                out_t = outputs.get(r)
+                if out_t is None:
+                    out_t = torch.empty(out_chunks * chunk, dtype=dtype, device=t_in.device)
+                out_ptr, out_elems = out_t.data_ptr(), out_t.numel()
+                if out_elems < written * chunk:
+                    raise PlanError(f'rank {r}: output of {out_elems} elements, program writes {written * chunk}')
+                results[r] = out_t
+            else:
+                results[r] = t_in
+            if scratch_chunks:
+                need = scratch_chunks * chunk * esize
+                scratch_t = plan.scratch.get(r)
+                if scratch_t is None or scratch_t.numel() < need:
+                    scratch_t = plan.scratch[r] = self._new_scratch(plan, r, need, t_in.device, direct)
+                scratch_ptr, scratch_elems = scratch_t.data_ptr(), scratch_t.numel() // esize
+            bits |= in_ptr | out_ptr | scratch_ptr
+            words += addresses
+            words += (in_ptr, out_ptr, scratch_ptr, in_elems, out_elems, scratch_elems)
+        if bits % esize:
+            raise PlanError('buffers must be aligned to their element size')
+        width = access_width(chunk, esize, (bits,))
+        proto = plan.host.proto
+        if proto == 2 and width != 16:
+            proto = 1                         # LL128 lines need 16-byte chunks; such calls run on the LL packets
+        geometry = self._one_gpu_geometry(plan, chunk, dtype, esize, width, proto, direct)
+        self.last_direct_mask = 7 if direct else 0
+        comm.native.launch_one_gpu(plan.dev_tbs, plan.dev_steps, comm.one_gpu_table.pack(*words), chunk, geometry, plan.grid,
+                                   DTYPE_CODES[dtype], proto, width, comm.timeout_ns, self.last_direct_mask,
+                                   (stream or torch.cuda.current_stream()).cuda_stream, self.cooperative, 0, 0)
         self.launches += 1
         return results
 

@@ -63,6 +63,7 @@ class HostPlan:
     direct_steps: int = 0          # send steps that may store straight into the receiver's slot
     eager_tbs: int = 0             # threadblocks whose receives are all opened at kernel start
     batched_steps: int = 0         # `re` steps folded into a multi-input add
+    single_hop: bool = False       # every tile is stored straight into its final slot and no step waits for another's tile
 
     def total_tbs(self):
         return sum(self.num_tbs[r] for r in self.local_ranks)
@@ -356,6 +357,7 @@ def compile_plan(algo: AlgoIR, local_ranks, slot_bytes: int, check=True, direct=
     opens = _open_positions(algo, match) if match else {}
     for r in range(algo.ngpus):
         plan.direct_bufs[r] = set()
+    plan.single_hop = simple
     stride = K_FIFO_SLOTS * slot_bytes
     tb_blob, step_blob = [], []
     nsteps_total = 0
@@ -413,6 +415,9 @@ def compile_plan(algo: AlgoIR, local_ranks, slot_bytes: int, check=True, direct=
                         if algo.gpus[pr].tbs[pt].steps[ps].cnt == st.cnt:
                             flags |= SF_DIRECT_RECV
                             plan.direct_bufs[rank].add(dbuf)
+                if st.type not in ('s', 'r', 'cpy') or st.depid >= 0 or (st.type == 's' and (
+                        not flags & SF_DIRECT_ALWAYS or any(x.type == 'r' for x in tb.steps[:si]))):
+                    plan.single_hop = False
                 nb = batches.get(si, 0)
                 if nb:
                     plan.batched_steps += sum(1 for k in range(si, si + nb) if tb.steps[k].type == 're')
@@ -450,38 +455,53 @@ def access_width(chunk_elems: int, elem_size: int, pointers=()):
     return elem_size
 
 
-# One-GPU interpreter (csrc/exec_one_gpu.cu).  SLICE_BYTES: a CTA's share of a chunk below which another slice only adds
-# flags.  TILE_BYTES: what a CTA moves between two signals of the Simple protocol.
-ONE_GPU_SLICE_BYTES = 4 << 10
+# One-GPU interpreter (csrc/exec_one_gpu.cu).  SLICE_BYTES: a CTA's share of a chunk below which another CTA only adds
+# flags (all-reduce of 1 MB over 8 ranks, LL128: 31 us with 4 KB, 29 with 16 KB).  TILE_BYTES: what a slice moves between
+# two signals of the Simple protocol; a hop costs a few microseconds beside the movement (256 MB ring all-reduce over 8
+# ranks, four slices per CTA: 1.90 ms with 32 KB, 1.56 with 64 KB, 1.52 with 128 KB).  STREAMS: 2.35 ms with one slice per
+# CTA, 1.77 with two, 1.52 with four, 1.53 with eight.
+ONE_GPU_SLICE_BYTES = 16 << 10
 ONE_GPU_TILE_BYTES = 128 << 10
+ONE_GPU_STREAMS = 4
+K_ONE_GPU_CHANNELS = 1024       # channels x slices that have flags of their own (csrc/msccl_device.h)
+K_ONE_GPU_PROGRESS = 4096       # threadblocks of a rank x slices
 
 
-def one_gpu_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_bytes: int, width: int, proto: int, max_ctas: int):
-    """(slices, slice_elems, tile_elems, slice_slot_bytes) of a launch with every rank on one GPU.
+def one_gpu_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_bytes: int, width: int, proto: int, max_ctas: int,
+                     direct=True):
+    """(CTAs per threadblock, slices per CTA, slice_elems, tile_elems, slot bytes of a slice) of a launch with every rank
+    on one GPU.
 
-    Each chunk is cut into ``slices`` parts of ``slice_elems`` elements (whole 128-byte lines), one CTA of every threadblock
-    per part: as many as fit on the GPU at once, have flags of their own (channels x slices, threadblocks x slices) and
-    are worth a CTA.  A slice moves in tiles of ``tile_elems`` through FIFO slots of ``slice_slot_bytes``."""
+    Each chunk is cut into slices of ``slice_elems`` elements (whole 128-byte lines) that run independently of each
+    other: as many CTAs per threadblock as fit on the GPU at once, have flags of their own and are worth a CTA, and under
+    the Simple protocol up to four slices per CTA as long as each has a whole tile.  A slice moves in tiles of
+    ``tile_elems`` through its own FIFO slots; in one tile when every tile is stored straight into its final slot and no
+    step waits for it (all-to-all of 32 MB: 153 us in tiles of 128 KB, 141 whole)."""
     per_access = width // elem_size
     if (chunk_elems * elem_size) % width:
         raise PlanError(f'chunks of {chunk_elems * elem_size} bytes are not whole {width}-byte accesses')
     tbs = max(plan.total_tbs(), 1)
     chans = 1 + max((tb.chan for g in plan.algo.gpus for tb in g.tbs), default=0)
     fifo_bytes = {0: width, 1: 32 if width == 16 else 8, 2: 128}[proto]          # one access (LL128: one line) in the FIFO
-    most = min(max_ctas // tbs, K_MAX_CHANNELS // chans, K_MAX_TBS // max(plan.algo.max_tbs_per_gpu(), 1),
-               slot_bytes // max(1024, 128 * -(-plan.max_cnt * fifo_bytes // 128)), -(-chunk_elems * elem_size // ONE_GPU_SLICE_BYTES))
-    slices = max(1, most)
+    least_slot = max(1024, 128 * -(-plan.max_cnt * fifo_bytes // 128))
+    most = min(K_ONE_GPU_CHANNELS // chans, K_ONE_GPU_PROGRESS // max(plan.algo.max_tbs_per_gpu(), 1), slot_bytes // least_slot)
+    chunk_bytes = chunk_elems * elem_size
+    ctas = max(1, min(max_ctas // tbs, most, -(-chunk_bytes // ONE_GPU_SLICE_BYTES)))
+    streams = 1
+    while proto == 0 and not (plan.single_hop and direct) and streams < ONE_GPU_STREAMS and 2 * streams * ctas <= most and \
+            chunk_bytes >= 2 * streams * ctas * ONE_GPU_TILE_BYTES:
+        streams *= 2
     line = max(per_access, 128 // elem_size)
-    slice_elems = -(-(-(-chunk_elems // slices)) // line) * line
-    slices = max(1, -(-chunk_elems // slice_elems))
-    slot = slot_bytes // slices // 128 * 128
+    slice_elems = -(-(-(-chunk_elems // (ctas * streams))) // line) * line
+    ctas = max(1, -(-chunk_elems // (slice_elems * streams)))
+    slot = slot_bytes // (ctas * streams) // 128 * 128
     if proto == 2:
         tile = slot // 128 // plan.max_cnt * 15 // 2 * per_access                # 15 units of 8 bytes per line
     else:
         tile = slot // (plan.max_cnt * fifo_bytes) * per_access
     if tile <= 0:
         raise PlanError('FIFO slot too small for this program')
-    if proto == 0:
+    if proto == 0 and not (plan.single_hop and direct):
         want = max(per_access, ONE_GPU_TILE_BYTES // plan.max_cnt // elem_size // line * line)
         want = max(want, -(-slice_elems // (K_MAX_ITERATIONS - 1) // per_access + 1) * per_access)
         tile = min(tile, want)
@@ -489,7 +509,7 @@ def one_gpu_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_byte
     if -(-slice_elems // tile) >= K_MAX_ITERATIONS:
         raise PlanError(f'{-(-slice_elems // tile)} iterations through FIFO slots of {slot} bytes exceed the executor limit '
                         f'of {K_MAX_ITERATIONS}: use a larger FIFO area')
-    return slices, slice_elems, tile, slot
+    return ctas, streams, slice_elems, tile, slot
 
 
 def tile_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_bytes: int, width: int = 16, proto=None):

@@ -51,13 +51,15 @@ def test_folded_chains_round_like_the_program(name, ranks, instances):
 @pytest.mark.parametrize('proto', [0, 1, 2])
 @pytest.mark.parametrize('max_ctas', [32, 148, 592])
 def test_one_gpu_geometry_covers_the_chunk(chunk, esize, proto, max_ctas):
-    plan = P.compile_plan(_program('two_shot', 4, 2, protocol='LL'), range(4), 64 << 10)
+    plan = P.compile_plan(_program('two_shot', 4, 2, protocol='LL'), range(4), 256 << 10)
     width = P.access_width(chunk, esize)
     proto = 1 if proto == 2 and width != 16 else proto
-    slices, slice_elems, tile, slot = P.one_gpu_geometry(plan, chunk, esize, 64 << 10, width, proto, max_ctas)
-    assert slices * plan.total_tbs() <= max_ctas and (slices - 1) * slice_elems < chunk <= slices * slice_elems
+    ctas, streams, slice_elems, tile, slot = P.one_gpu_geometry(plan, chunk, esize, 256 << 10, width, proto, max_ctas)
+    slices = ctas * streams
+    assert ctas * plan.total_tbs() <= max_ctas and (streams == 1 or proto == 0)
+    assert (ctas - 1) * streams * slice_elems < chunk <= slices * slice_elems
     assert slice_elems * esize % width == 0 and 0 < tile <= slice_elems and tile * esize % width == 0
-    assert slot % 128 == 0 and slot * slices <= 64 << 10
+    assert slot % 128 == 0 and slot * slices <= 256 << 10
     accesses = tile * esize // width
     fifo = {0: accesses * width, 1: accesses * (32 if width == 16 else 8), 2: -(-2 * accesses // 15) * 128}[proto]
     assert fifo * plan.max_cnt <= slot
