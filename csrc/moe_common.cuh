@@ -117,10 +117,10 @@ __device__ __forceinline__ bool load_counts(const MoeArgs& g, FusedPage* page, u
   return *abort_flag == 0;
 }
 
-// The comm CTAs of the dispatch kernel (the first g.comm_ctas CTAs of the grid): all-gather the per-expert counts,
+// The comm CTAs of the dispatch kernel (the first `ctas` CTAs of the grid): all-gather the per-expert counts,
 // then scatter my token copies into the owners' dispatch buffers and publish one flag per destination.
 __device__ __forceinline__ void moe_comm_role(const MoeArgs& g, FusedPage* page, unsigned long long epoch, int parity, MoeShared* sh,
-                                          volatile int* abort_flag) {
+                                          volatile int* abort_flag, int ctas) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int copies = g.tokens * g.topk;
   const size_t row_bytes = static_cast<size_t>(g.hidden) * 2;
@@ -140,7 +140,7 @@ __device__ __forceinline__ void moe_comm_role(const MoeArgs& g, FusedPage* page,
   if (!load_counts(g, page, epoch, parity, sh, abort_flag)) return;
   {
     // scatter rows: one warp per token copy, copies taken in expert order
-    const int warps = g.comm_ctas * (kGemmThreads / 32);
+    const int warps = ctas * (kGemmThreads / 32);
     const int gw = blockIdx.x * (kGemmThreads / 32) + warp;
     for (int i = gw; i < copies; i += warps) {
       const int c = g.sorted_copy[i];
@@ -176,7 +176,7 @@ __device__ __forceinline__ void moe_comm_role(const MoeArgs& g, FusedPage* page,
     __syncthreads();
     if (threadIdx.x == 0) {
       fence_acq_rel_sys();
-      if (atomicAdd(&page->ag_block_count[0], 1u) == static_cast<unsigned int>(g.comm_ctas) - 1u) {
+      if (atomicAdd(&page->ag_block_count[0], 1u) == static_cast<unsigned int>(ctas) - 1u) {
         page->ag_block_count[0] = 0;
         fence_acq_rel_sys();
         for (int q = 0; q < g.nranks; ++q) st_release_sys(&g.pages[(g.rank + q) % g.nranks]->moe_flag[g.rank][1], epoch);
