@@ -280,17 +280,20 @@ int max_cta_pairs(int epilogue) {
   return clusters;
 }
 
-// Same contract as gemm_bf16 with bn = 256; N % 256 == 0, K % 64 == 0.
+// Same contract as gemm_bf16 with bn = 256; N % 256 == 0, K % 64 == 0.  `split`: the sum over K may be formed in parts
+// (gemm_splitk_sm100.cu) when the tiles would leave most of the GPU idle.
 cudaError_t gemm_bf16_2cta(const void* a, const void* b, void* d, int M, int N, int K, int lda, int ldb, int ldd, int epilogue,
-                           int* error_words, int max_pairs, cudaStream_t stream) {
+                           int* error_words, int max_pairs, cudaStream_t stream, bool split) {
   if (K % BK != 0 || N % PBN != 0 || M <= 0) return cudaErrorInvalidValue;
+  const CUtensorMap map_a = make_bf16_kmajor_map(a, M, K, lda, BM);
+  const CUtensorMap map_b = make_bf16_kmajor_map(b, N, K, ldb, PBN / 2);
+  const int ways = split && max_pairs <= 0 ? splitk_ways(M, N, K, epilogue) : 1;
+  if (ways > 1) return gemm_bf16_splitk(map_a, map_b, d, M, N, K, ldd, epilogue, error_words, ways, stream);
   int pairs = max_cta_pairs(epilogue);
   if (pairs <= 0) return cudaErrorLaunchOutOfResources;
   if (max_pairs > 0 && max_pairs < pairs) pairs = max_pairs;
   const int tiles = ((M + PBM - 1) / PBM) * (N / PBN);
   if (tiles < pairs) pairs = tiles;
-  CUtensorMap map_a = make_bf16_kmajor_map(a, M, K, lda, BM);
-  CUtensorMap map_b = make_bf16_kmajor_map(b, N, K, ldb, PBN / 2);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(kGemmThreads, 1, 1);

@@ -50,7 +50,8 @@ def interleave_gate_up(w_gate, w_up, tile=256):
 def gemm_bf16(a, b, out=None, epilogue='none', bn=256, max_ctas=0, stream=None, pair=None):
     """``a``: [M, K] bf16, ``b``: [N, K] bf16 (row pitch may exceed K).  Returns [M, N] (or [M, N/2] for swiglu).
     ``pair``: run on CTA pairs (``tcgen05 cta_group::2``, 256 x 256 tiles; needs N % 256 == 0); ``None`` takes
-    ``MSCCL_GEMM_PAIR`` (default on) whenever the shape allows it and ``bn`` is 256."""
+    ``MSCCL_GEMM_PAIR`` (default on) whenever the shape allows it and ``bn`` is 256, and for few tiles splits K over the
+    pairs of a cluster (``csrc/gemm_splitk_sm100.cu``)."""
     assert a.is_cuda and b.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
     m, k = a.shape
@@ -64,13 +65,14 @@ def gemm_bf16(a, b, out=None, epilogue='none', bn=256, max_ctas=0, stream=None, 
         out = torch.empty(m, n_out, dtype=torch.bfloat16, device=a.device)
     assert out.shape == (m, n_out) and out.stride(1) == 1 and out.dtype == torch.bfloat16
     stream_h = (stream or torch.cuda.current_stream()).cuda_stream
+    split = pair is None            # an explicit choice of kernel also fixes the order of the sums
     if pair is None:
         pair = bn == 256 and n % 256 == 0 and os.environ.get('MSCCL_GEMM_PAIR', '1') == '1'
     if pair:
         if n % 256:
             raise ValueError(f'the two-CTA kernel needs N to be a multiple of 256 (got {n})')
         load().gemm_bf16_2cta(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
-                              1 if swiglu else 0, _errors(a.device).data_ptr(), (max_ctas + 1) // 2, stream_h)
+                              1 if swiglu else 0, _errors(a.device).data_ptr(), (max_ctas + 1) // 2, stream_h, split)
         return out
     load().gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, a.stride(0), b.stride(0), out.stride(0),
                      1 if swiglu else 0, bn, _errors(a.device).data_ptr(), max_ctas, stream_h)

@@ -1,0 +1,38 @@
+"""GEMM paths chosen by shape: K split over the pairs of a cluster."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(m, n, k, seed=0):
+    gen = torch.Generator(device='cuda').manual_seed(seed)
+    a = torch.randn(m, k, device='cuda', generator=gen).bfloat16()
+    b = (torch.randn(n, k, device='cuda', generator=gen) * 0.05).bfloat16()
+    return a, b
+
+
+def _close(d, want):
+    # one rounding to bf16 (2^-9 of the value) on top of fp32 sums (a few 1e-6 of the largest); twice that
+    assert torch.all((d.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max())
+
+
+def _swiglu(full):
+    t = full.view(full.shape[0], -1, 2, 128)
+    return (torch.nn.functional.silu(t[:, :, 0]) * t[:, :, 1]).reshape(full.shape[0], -1)
+
+
+@pytest.mark.parametrize('m,n,k', [(1, 256, 1024), (128, 256, 512), (129, 512, 576), (256, 3584, 4096), (256, 4096, 1792), (300, 1024, 1088),
+                                   (257, 4096, 8192), (512, 4352, 1024), (16, 256, 64)])
+def test_split_k_matches_the_unsplit_product(m, n, k):
+    from msccl.ops import check_gemm_errors, gemm_bf16
+    a, b = _operands(m, n, k)
+    full = a.double() @ b.double().t()
+    _close(gemm_bf16(a, b), full)
+    _close(gemm_bf16(a, b, epilogue='swiglu'), _swiglu(full))
+    check_gemm_errors()
+    # rows beyond M and columns beyond the result are left alone
+    holder = torch.full((m + 2, n + 64), 7.0, device='cuda', dtype=torch.bfloat16)
+    gemm_bf16(a, b, out=holder[1:m + 1, :n])
+    assert torch.all(holder[0] == 7) and torch.all(holder[m + 1] == 7) and torch.all(holder[1:, n:] == 7)
+    _close(holder[1:m + 1, :n], full)
