@@ -21,6 +21,7 @@
 #include "gemm_sm100.cuh"
 #include "gemm_sm100.h"
 #include "mxfp8_pair.cuh"
+#include "quantize_mx.cuh"
 #include "umma_2cta.cuh"
 
 namespace msccl {
@@ -28,10 +29,18 @@ namespace sm100 {
 
 namespace {
 
-__global__ void __launch_bounds__(kGemmThreads, 1)
+// EPI 0: bf16 result.  EPI 1: SwiGLU over the tile's (gate | up) column halves, rounded to bf16 and quantised again - the
+// operand of the next block-scaled GEMM leaves the kernel ready (d: e4m3 values with a pitch of ldd bytes, sf_out: scale
+// blocks).  Two warps share a lane quarter there: each takes its 2 x 64 columns out of tensor memory in one go and frees the
+// accumulator before it computes anything.
+template <int EPI>
+constexpr int kMxThreads = EPI == 0 ? kGemmThreads : kGemmThreads + 128;
+
+template <int EPI>
+__global__ void __launch_bounds__(kMxThreads<EPI>, 1)
 gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
-                       __nv_bfloat16* __restrict__ d, int M, int N, int K, int ldd, int* error_words) {
+                       void* __restrict__ d_out, uint8_t* __restrict__ sf_out, int M, int N, int K, int ldd, int* error_words) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* stage_base = smem;
@@ -39,7 +48,7 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   uint64_t* full_bar = bars;                         // leader only: loads of both CTAs complete here
   uint64_t* empty_bar = bars + kQStages;             // per CTA: commit from the leader
   uint64_t* acc_full = bars + 2 * kQStages;          // per CTA: commit from the leader
-  uint64_t* acc_empty = bars + 2 * kQStages + 1;     // leader only: 8 epilogue warps of the pair
+  uint64_t* acc_empty = bars + 2 * kQStages + 1;     // leader only: the epilogue warps of the pair
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kQStages + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint8_t* epi_base = smem + static_cast<size_t>(kQStages) * kQStageBytes + 256;
@@ -60,7 +69,7 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(acc_full, 1);
-    mbar_init(acc_empty, 8);
+    mbar_init(acc_empty, EPI == 0 ? 8 : 16);        // the epilogue warps of both CTAs
     *abort_flag = 0;
     mbar_fence_init();
     prefetch_tensormap(&map_a);
@@ -164,7 +173,8 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
     }
   } else {
-    // ---------------------------------------------------------------- epilogue (warps 2..5, both CTAs)
+    // ---------------------------------------------------------------- epilogue (warps 2.., both CTAs)
+    __nv_bfloat16* const d = static_cast<__nv_bfloat16*>(d_out);
     const int quarter = warp % 4;
     uint32_t acc_phase = 0;
     for (int tile = first_tile; tile < num_tiles; tile += tile_step) {
@@ -179,6 +189,45 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       tc_fence_after_sync();
       const int row0 = tm * QBM + static_cast<int>(cta_rank) * BM + quarter * 32;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+      if constexpr (EPI == 1) {
+        constexpr int H = QBN / 2;
+        const int c0 = (warp - 2) / 4 * (H / 2);       // this warp's 64 gate columns and the 64 up columns beside them
+        uint32_t gt[2][32], up[2][32];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          tmem_ld32(taddr + c0 + 32 * i, gt[i]);
+          tmem_ld32(taddr + H + c0 + 32 * i, up[i]);
+        }
+        tc_wait_ld();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(acc_empty), 0));
+        const int row = row0 + lane;
+        uint32_t scales = 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float v[32];
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const float gv = __uint_as_float(gt[i][e]);
+            v[e] = __bfloat162float(__float2bfloat16_rn(gv / (1.0f + __expf(-gv)) * __uint_as_float(up[i][e])));
+          }
+          uint32_t packed[8];
+          scales |= static_cast<uint32_t>(quantize_mx_group(v, packed) + 127) << (8 * i);
+          if (row < M) {
+            uint4* out = reinterpret_cast<uint4*>(static_cast<uint8_t*>(d_out) + static_cast<size_t>(row) * ldd + tn * H + c0 + 32 * i);
+            out[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            out[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+          }
+        }
+        if (row < M) {                                 // block (row / 128, tn), see quantize_mx.cu; two of its row's four scales
+          const int r = row % 128;
+          *reinterpret_cast<uint16_t*>(sf_out + (static_cast<size_t>(row / 128) * tiles_n + tn) * 512 + (r % 32) * 16 + (r / 32) * 4 +
+                                       c0 / 32) = static_cast<uint16_t>(scales);
+        }
+        acc_phase ^= 1;
+        continue;
+      }
       uint8_t* epi = epi_base + (warp - 2) * kQEpiPerWarp;
       constexpr int kLanesPerRow = kQStageCols * 2 / 16, kRowsPerStore = 32 / kLanesPerRow;
 #pragma unroll 1
@@ -237,27 +286,14 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   }
 }
 
+template <int EPI>
 int max_pairs_mxfp8() {
   static int cached[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && cached[dev] > 0) return cached[dev];
-  if (cudaFuncSetAttribute(gemm_mxfp8_2cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kQSmemBytes)) !=
-      cudaSuccess)
-    return 0;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * sm_count(), 1, 1);
-  cfg.blockDim = dim3(kGemmThreads, 1, 1);
-  cfg.dynamicSmemBytes = kQSmemBytes;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_mxfp8_2cta_kernel, &cfg) != cudaSuccess) {
+  if (pair_clusters(gemm_mxfp8_2cta_kernel<EPI>, kQSmemBytes, &clusters, kMxThreads<EPI>) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -265,37 +301,40 @@ int max_pairs_mxfp8() {
   return clusters;
 }
 
-}  // namespace
-
-// Same contract as gemm_mxfp8; N % 256 == 0, K % 128 == 0.  The packed A scales must cover a multiple
-// of 256 rows (pack_mx_scales pads to 128; the caller passes ceil(M / 256) * 2 row blocks).
-cudaError_t gemm_mxfp8_2cta(const void* a, const void* sfa, const void* b, const void* sfb, void* d, int M, int N, int K, int lda,
-                            int ldb, int ldd, int* error_words, int max_pairs, cudaStream_t stream) {
+template <int EPI>
+cudaError_t launch(const void* a, const void* sfa, const void* b, const void* sfb, void* d, void* sf_out, int M, int N, int K, int lda,
+                   int ldb, int ldd, int* error_words, int max_pairs, cudaStream_t stream) {
   if (K % QBK != 0 || N % QBN != 0 || M <= 0) return cudaErrorInvalidValue;
   if (reinterpret_cast<uintptr_t>(sfa) % 16 != 0 || reinterpret_cast<uintptr_t>(sfb) % 16 != 0) return cudaErrorInvalidValue;
-  int pairs = max_pairs_mxfp8();
+  int pairs = max_pairs_mxfp8<EPI>();
   if (pairs <= 0) return cudaErrorLaunchOutOfResources;
   if (max_pairs > 0 && max_pairs < pairs) pairs = max_pairs;
   const int tiles = ((M + QBM - 1) / QBM) * (N / QBN);
   if (tiles < pairs) pairs = tiles;
-  CUtensorMap map_a = make_u8_kmajor_map(a, M, K, lda, BM);
-  CUtensorMap map_b = make_u8_kmajor_map(b, N, K, ldb, QBN / 2);
-  CUtensorMap map_sfa = make_block512_map(sfa, static_cast<uint64_t>((M + QBM - 1) / QBM) * 2 * (K / QBK));
-  CUtensorMap map_sfb = make_block512_map(sfb, static_cast<uint64_t>(N / 128) * (K / QBK));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs, 1, 1);
-  cfg.blockDim = dim3(kGemmThreads, 1, 1);
-  cfg.dynamicSmemBytes = kQSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_mxfp8_2cta_kernel, map_a, map_b, map_sfa, map_sfb, static_cast<__nv_bfloat16*>(d), M, N, K,
-                            ldd, error_words);
+  const CUtensorMap map_a = make_u8_kmajor_map(a, M, K, lda, BM);
+  const CUtensorMap map_b = make_u8_kmajor_map(b, N, K, ldb, QBN / 2);
+  // behind an odd last 128-row block the pair's second CTA reads scales (and rows) past the end, which are zeros
+  const CUtensorMap map_sfa = make_block512_map(sfa, static_cast<uint64_t>((M + BM - 1) / BM) * (K / QBK));
+  const CUtensorMap map_sfb = make_block512_map(sfb, static_cast<uint64_t>(N / 128) * (K / QBK));
+  return launch_pairs_threads(gemm_mxfp8_2cta_kernel<EPI>, kQSmemBytes, pairs, kMxThreads<EPI>, stream, map_a, map_b, map_sfa, map_sfb, d,
+                              static_cast<uint8_t*>(sf_out), M, N, K, ldd, error_words);
+}
+
+}  // namespace
+
+// Same contract as gemm_mxfp8; N % 256 == 0, K % 128 == 0. 
+cudaError_t gemm_mxfp8_2cta(const void* a, const void* sfa, const void* b, const void* sfb, void* d, int M, int N, int K, int lda,
+                            int ldb, int ldd, int* error_words, int max_pairs, cudaStream_t stream) {
+  return launch<0>(a, sfa, b, sfb, d, nullptr, M, N, K, lda, ldb, ldd, error_words, max_pairs, stream);
+}
+
+// SwiGLU of the product, quantised: q is [M, N / 2] e4m3 with a pitch of ldq bytes, sf_out its scale blocks (the rows
+// beyond M inside the last one are not written).  B's rows interleave 128 gate rows and the 128 up rows of the same features.
+cudaError_t gemm_mxfp8_swiglu_2cta(const void* a, const void* sfa, const void* b, const void* sfb, void* q, void* sf_out, int M, int N,
+                                   int K, int lda, int ldb, int ldq, int* error_words, int max_pairs, cudaStream_t stream) {
+  if (ldq % 16 != 0 || reinterpret_cast<uintptr_t>(q) % 16 != 0 || reinterpret_cast<uintptr_t>(sf_out) % 16 != 0)
+    return cudaErrorInvalidValue;
+  return launch<1>(a, sfa, b, sfb, q, sf_out, M, N, K, lda, ldb, ldq, error_words, max_pairs, stream);
 }
 
 }  // namespace sm100

@@ -29,10 +29,12 @@ cudaError_t gemm_bf16_splitk(const CUtensorMap& map_a, const CUtensorMap& map_b,
 // Block-scaled fp8 (e4m3 with one UE8M0 scale per 32 K elements), see gemm_mxfp8_sm100.cu.
 cudaError_t gemm_mxfp8(const void* a, const void* sfa, const void* b, const void* sfb, void* d, int M, int N, int K, int lda,
                        int ldb, int ldd, int* error_words, int max_ctas, cudaStream_t stream);
-// The same on CTA pairs with 256 x 256 tiles (gemm_mxfp8_2cta_sm100.cu).  N % 256 == 0; sfa must hold an even
-// number of 128-row blocks (2 * ceil(M / 256)).
+// The same on CTA pairs with 256 x 256 tiles (gemm_mxfp8_2cta_sm100.cu).  N % 256 == 0.
 cudaError_t gemm_mxfp8_2cta(const void* a, const void* sfa, const void* b, const void* sfb, void* d, int M, int N, int K, int lda,
                             int ldb, int ldd, int* error_words, int max_pairs, cudaStream_t stream);
+// ... with a SwiGLU epilogue whose result is quantised to the same format.
+cudaError_t gemm_mxfp8_swiglu_2cta(const void* a, const void* sfa, const void* b, const void* sfb, void* q, void* sf_out, int M, int N,
+                                   int K, int lda, int ldb, int ldq, int* error_words, int max_pairs, cudaStream_t stream);
 
 }  // namespace sm100
 }  // namespace msccl

@@ -4,10 +4,11 @@
 // for K elements [32 j, 32 j + 32)).  One thread owns one group of 32 elements: 64 bytes in, 32 bytes + 1 byte out.
 // The scale is the smallest power of two that brings the group's largest magnitude inside the e4m3 range (448).
 #include <cuda_bf16.h>
-#include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
+
+#include "quantize_mx.cuh"
 
 namespace msccl {
 namespace sm100 {
@@ -34,23 +35,8 @@ __global__ void __launch_bounds__(256) quantize_mx_kernel(const __nv_bfloat16* _
       v[8 * i + 2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
     }
   }
-  float amax = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
-  amax = fmaxf(amax, 1.0e-36f);
-  // smallest e with amax / 2^e <= 448
-  const float ratio = amax / 448.0f;
-  int e = ilogbf(ratio);
-  if (ldexpf(1.0f, e) < ratio) ++e;
-  e = max(-127, min(127, e));
-  const float inv = ldexpf(1.0f, -e);
   uint32_t packed[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * i] * inv, v[4 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-    const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * i + 2] * inv, v[4 * i + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-    packed[i] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
-  }
+  const int e = quantize_mx_group(v, packed);
   uint4* dst = reinterpret_cast<uint4*>(q + static_cast<long long>(row) * K + grp * 32);
   dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
   dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);

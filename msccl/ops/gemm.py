@@ -144,7 +144,7 @@ def gemm_mxfp8(a, sfa_packed, b, sfb_packed, out=None, max_ctas=0, stream=None, 
     """``a``: [M, K] e4m3, ``b``: [N, K] e4m3, scales packed by ``pack_mx_scales``.  Returns bf16 [M, N] =
     dequant(a) @ dequant(b).T with the scaling done inside the tensor core (tcgen05 block_scale MMA).
     ``pair``: CTA pairs with 256 x 256 tiles (needs N % 256 == 0 and A scales padded to 256 rows);
-    ``None`` uses them whenever the operands allow it (``MSCCL_GEMM_PAIR=0`` turns that off)."""
+    ``None`` uses them whenever N allows it (``MSCCL_GEMM_PAIR=0`` turns that off)."""
     assert a.is_cuda and b.is_cuda and a.dtype == torch.float8_e4m3fn and b.dtype == torch.float8_e4m3fn
     assert a.dim() == 2 and b.dim() == 2 and a.stride(1) == 1 and b.stride(1) == 1
     m, k = a.shape
@@ -158,8 +158,9 @@ def gemm_mxfp8(a, sfa_packed, b, sfb_packed, out=None, max_ctas=0, stream=None, 
         raise ValueError(f'packed scales must hold {need_a} (or {need_a_pair}) and {need_b} bytes')
     can_pair = n % 256 == 0 and sfa_packed.numel() == need_a_pair
     if pair is None:
-        pair = can_pair and os.environ.get('MSCCL_GEMM_PAIR', '1') == '1'
-    if pair and not can_pair:
+        # scales padded to 128 rows do as well: behind an odd last block the second CTA of a pair reads zeros
+        pair = n % 256 == 0 and os.environ.get('MSCCL_GEMM_PAIR', '1') == '1'
+    elif pair and not can_pair:
         raise ValueError('the CTA-pair kernel needs N % 256 == 0 and A scales packed with row_multiple=256')
     assert sfa_packed.dtype == torch.uint8 and sfb_packed.dtype == torch.uint8 and sfa_packed.is_contiguous()
     if out is None:
@@ -174,3 +175,19 @@ def gemm_mxfp8(a, sfa_packed, b, sfb_packed, out=None, max_ctas=0, stream=None, 
     load().gemm_mxfp8(a.data_ptr(), sfa_packed.data_ptr(), b.data_ptr(), sfb_packed.data_ptr(), out.data_ptr(), m, n, k,
                       a.stride(0), b.stride(0), out.stride(0), _errors(a.device).data_ptr(), max_ctas, stream_h)
     return out
+
+
+def gemm_mxfp8_swiglu(a, sfa_packed, b, sfb_packed, out, scales_out, stream=None):
+    """``silu(gate) * up`` of ``dequant(a) @ dequant(b).T``, quantised for the next GEMM: the same bytes as
+    ``quantize_mxfp8_packed`` gives for the bf16 result, without the trip through memory (8192 x 28672 x 4096: 235 MB written
+    and read again).  ``b``: ``interleave_gate_up(..., tile=256)``; ``out`` [M, N / 2] e4m3 and ``scales_out`` are filled."""
+    m, k = a.shape
+    n = b.shape[0]
+    assert a.dtype == b.dtype == out.dtype == torch.float8_e4m3fn and a.stride(1) == b.stride(1) == 1 and out.is_contiguous()
+    assert b.shape[1] == k and k % 128 == 0 and n % 256 == 0 and out.shape == (m, n // 2)
+    assert sfa_packed.numel() >= -(-m // 128) * (k // 128) * 512 and sfb_packed.numel() >= (n // 128) * (k // 128) * 512
+    assert scales_out.dtype == torch.uint8 and scales_out.numel() == -(-m // 128) * (n // 256) * 512
+    load().gemm_mxfp8_swiglu_2cta(a.data_ptr(), sfa_packed.data_ptr(), b.data_ptr(), sfb_packed.data_ptr(), out.data_ptr(),
+                                  scales_out.data_ptr(), m, n, k, a.stride(0), b.stride(0), n // 2, _errors(a.device).data_ptr(),
+                                  (stream or torch.cuda.current_stream()).cuda_stream)
+    return out, scales_out

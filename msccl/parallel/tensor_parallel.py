@@ -6,11 +6,18 @@
 ``precision='mxfp8'`` runs both kernels on block-scaled fp8 operands (OCP MX: e4m3 values, one power-of-two scale per
 32 K elements): the weights are quantised once, the activations per call (the token shard before the all-gather, the
 SwiGLU output before the down projection); accumulation is fp32 and the result bf16 either way.
+
+With one rank there is nothing to gather or to scatter: the layer runs on the plain GEMM kernels, whose tiles have the whole
+GPU (the fused kernels set 8 and 12 SMs aside for the exchange) and walk the rows of a group first, so that activations stay
+in L2 while the weights stream.
 """
+import os
+
 import torch
 
 from msccl.ops.fused_tp import FusedTensorParallel
-from msccl.ops.gemm import interleave_gate_up, pack_mx_scales, quantize_mxfp8, quantize_mxfp8_packed
+from msccl.ops.gemm import (gemm_bf16, gemm_mxfp8, gemm_mxfp8_swiglu, interleave_gate_up, pack_mx_scales, quantize_mxfp8,
+                            quantize_mxfp8_packed)
 
 
 class TensorParallelMLP:
@@ -31,8 +38,13 @@ class TensorParallelMLP:
         self.w_down = mk(hidden, self.shard) if w_down is None else w_down.contiguous()
         self.fused = FusedTensorParallel(comm, tokens_per_rank, hidden)
         self.h = torch.empty(comm.world * tokens_per_rank, self.shard, dtype=torch.bfloat16, device=dev)
+        # MSCCL_FUSED_PAIR=0 asks for the fused single-CTA kernels whatever the number of ranks
+        self.plain = comm.world == 1 and os.environ.get('MSCCL_FUSED_PAIR', '1') != '0'
         if precision == 'mxfp8':
-            gu = interleave_gate_up(w_gate, w_up, tile=self.fused.mx_gate_up_tile)   # 256 on CTA pairs, 128 on single CTAs
+            if self.plain:
+                self.h_q = torch.empty(tokens_per_rank, self.shard, dtype=torch.float8_e4m3fn, device=dev)
+                self.h_sf = torch.empty(tokens_per_rank // 128 * (self.shard // 128) * 512, dtype=torch.uint8, device=dev)
+            gu = interleave_gate_up(w_gate, w_up, tile=256 if self.plain else self.fused.mx_gate_up_tile)   # 256 on CTA pairs
             self.wq_gate_up, s = quantize_mxfp8(gu.float())
             self.sf_gate_up = pack_mx_scales(s, row_multiple=128)
             self.wq_down, s = quantize_mxfp8(self.w_down.float())
@@ -40,6 +52,15 @@ class TensorParallelMLP:
 
     def forward(self, x_local, out=None):
         """x_local: [tokens_per_rank, hidden] -> this rank's [tokens_per_rank, hidden] of the MLP output."""
+        if self.plain:
+            assert x_local.shape == (self.fused.rows, self.fused.hidden) and x_local.is_contiguous() and x_local.dtype == torch.bfloat16
+            assert out is None or out.is_contiguous()
+            self.fused.launches += 2
+            if self.precision == 'mxfp8':
+                xq, sx = quantize_mxfp8_packed(x_local)
+                hq, sh = gemm_mxfp8_swiglu(xq, sx, self.wq_gate_up, self.sf_gate_up, self.h_q, self.h_sf)
+                return gemm_mxfp8(hq, sh, self.wq_down, self.sf_down, out=out)
+            return gemm_bf16(gemm_bf16(x_local, self.w_gate_up, out=self.h, epilogue='swiglu'), self.w_down, out=out)
         if self.precision == 'mxfp8':
             xq, sx = quantize_mxfp8_packed(x_local)                  # one kernel each: values + packed scales
             self.fused.all_gather_gemm_mxfp8(xq, sx, self.wq_gate_up, self.sf_gate_up, epilogue='swiglu', out=self.h)

@@ -1,4 +1,5 @@
-"""GEMM paths chosen by shape: K split over the pairs of a cluster."""
+"""GEMM paths chosen by shape: K split over the pairs of a cluster, odd row blocks on CTA pairs, and the block-scaled GEMM
+whose SwiGLU result leaves quantised."""
 import pytest
 import torch
 
@@ -36,3 +37,30 @@ def test_split_k_matches_the_unsplit_product(m, n, k):
     gemm_bf16(a, b, out=holder[1:m + 1, :n])
     assert torch.all(holder[0] == 7) and torch.all(holder[m + 1] == 7) and torch.all(holder[1:, n:] == 7)
     _close(holder[1:m + 1, :n], full)
+
+
+@pytest.mark.parametrize('m,n,k', [(1, 256, 128), (128, 512, 256), (130, 256, 1024), (384, 768, 1792), (640, 256, 128)])
+def test_block_scaled_gemm_on_pairs_behind_an_odd_row_block(m, n, k):
+    from msccl.ops import check_gemm_errors
+    from msccl.ops.gemm import gemm_mxfp8, quantize_mxfp8_packed
+    a, b = _operands(m, n, k, 1)
+    (aq, sa), (bq, sb) = quantize_mxfp8_packed(a), quantize_mxfp8_packed(b)
+    assert torch.equal(gemm_mxfp8(aq, sa, bq, sb), gemm_mxfp8(aq, sa, bq, sb, pair=False))
+    check_gemm_errors()
+
+
+@pytest.mark.parametrize('m,n,k', [(128, 256, 128), (256, 512, 512), (384, 1024, 256), (1024, 7168, 1024)])
+def test_quantised_swiglu_epilogue(m, n, k):
+    from msccl.ops import check_gemm_errors
+    from msccl.ops.gemm import dequantize_mxfp8, gemm_mxfp8_swiglu, quantize_mxfp8, quantize_mxfp8_packed
+    a, b = _operands(m, n, k, 2)
+    (aq, sa), (bq, sb) = quantize_mxfp8_packed(a), quantize_mxfp8_packed(b)
+    q = torch.empty(m, n // 2, dtype=torch.float8_e4m3fn, device='cuda')
+    sf = torch.full((m // 128 * (n // 256) * 512,), 255, dtype=torch.uint8, device='cuda')
+    gemm_mxfp8_swiglu(aq, sa, bq, sb, q, sf)
+    check_gemm_errors()
+    h = _swiglu((dequantize_mxfp8(*quantize_mxfp8(a.float())).double() @ dequantize_mxfp8(*quantize_mxfp8(b.float())).double().t()))
+    want_q, want_sf = quantize_mxfp8_packed(h.to(torch.bfloat16))
+    # a bf16 value on the other side of a rounding or e4m3 boundary may differ; nearly all bytes are the same
+    assert (q.view(torch.uint8) != want_q.view(torch.uint8)).float().mean() < 0.02
+    assert (sf != want_sf).float().mean() < 0.002
