@@ -54,13 +54,19 @@ class TensorParallelMLP:
         """x_local: [tokens_per_rank, hidden] -> this rank's [tokens_per_rank, hidden] of the MLP output."""
         if self.plain:
             assert x_local.shape == (self.fused.rows, self.fused.hidden) and x_local.is_contiguous() and x_local.dtype == torch.bfloat16
-            assert out is None or out.is_contiguous()
+            rows, hidden = x_local.shape
+            if out is None:
+                out = torch.empty(rows, hidden, dtype=torch.bfloat16, device=x_local.device)
+            assert out.is_contiguous()
+            y = out.view(-1).view(torch.bfloat16)[:rows * hidden].view(rows, hidden)      # any contiguous memory of that size will do
             self.fused.launches += 2
             if self.precision == 'mxfp8':
                 xq, sx = quantize_mxfp8_packed(x_local)
                 hq, sh = gemm_mxfp8_swiglu(xq, sx, self.wq_gate_up, self.sf_gate_up, self.h_q, self.h_sf)
-                return gemm_mxfp8(hq, sh, self.wq_down, self.sf_down, out=out)
-            return gemm_bf16(gemm_bf16(x_local, self.w_gate_up, out=self.h, epilogue='swiglu'), self.w_down, out=out)
+                gemm_mxfp8(hq, sh, self.wq_down, self.sf_down, out=y)
+            else:
+                gemm_bf16(gemm_bf16(x_local, self.w_gate_up, out=self.h, epilogue='swiglu'), self.w_down, out=y)
+            return out
         if self.precision == 'mxfp8':
             xq, sx = quantize_mxfp8_packed(x_local)                  # one kernel each: values + packed scales
             self.fused.all_gather_gemm_mxfp8(xq, sx, self.wq_gate_up, self.sf_gate_up, epilogue='swiglu', out=self.h)

@@ -1,0 +1,98 @@
+"""The one-GPU interpreter where it can go wrong: several CTAs and slices per threadblock, chunks and buffers at every
+alignment, reduces longer than one batch - bit for bit against the CPU interpreter."""
+import pytest
+import torch
+
+from msccl.interp import input_chunks_of, run_algorithm
+from msccl.language import MSCCLProgram, ThreadblockPolicy
+from msccl.language.collectives import AllGather, AllReduce, AllToAll, ReduceScatter
+from msccl.programs.allgather import allgather_direct, reduce_scatter_direct
+from msccl.programs.allreduce import allreduce_one_shot, allreduce_ring, allreduce_two_shot
+from msccl.programs.alltoall import alltoall_direct
+from msccl.topologies import fully_connected
+from msccl.xml import load_xml
+
+pytestmark = pytest.mark.gpu
+
+BODIES = {
+    'ring': (lambda n: AllReduce(n, n, True), lambda n: allreduce_ring(n, min(n, 2)), True),
+    'two_shot': (lambda n: AllReduce(n, n, True), allreduce_two_shot, True),
+    'one_shot': (lambda n: AllReduce(n, 1, True), allreduce_one_shot, True),
+    'allgather': (lambda n: AllGather(n, 1, False), allgather_direct, False),
+    'reduce_scatter': (lambda n: ReduceScatter(n, 1, False), reduce_scatter_direct, False),
+    'alltoall': (lambda n: AllToAll(n, 1, False), alltoall_direct, False),
+}
+
+
+def _algo(name, ranks, protocol):
+    coll, body, manual = BODIES[name]
+    policy = dict(threadblock_policy=ThreadblockPolicy.manual) if manual else {}
+    prog = MSCCLProgram(name, fully_connected(ranks), coll(ranks), 1, protocol=protocol, **policy)
+    with prog:
+        body(ranks)
+    return load_xml(prog.generate_xml())
+
+
+def _check(algo, chunk, dtype, misalign=0, fifo_bytes=8 << 20, direct='auto', tile=None, monkeypatch=None, streams=1):
+    from msccl.runtime import Communicator, Executor
+    import msccl.runtime.plan as P
+    if tile:
+        monkeypatch.setattr(P, 'ONE_GPU_TILE_BYTES', tile)
+    comm = Communicator.emulated(algo.ngpus, fifo_bytes=fifo_bytes)
+    try:
+        ex = Executor(comm)
+        plan = ex.compile(algo)
+        gen = torch.Generator().manual_seed(chunk)
+        host = [torch.randn(input_chunks_of(algo, r) * chunk, generator=gen).to(dtype) for r in range(algo.ngpus)]
+        want = run_algorithm(algo, host, chunk, dtype=dtype)
+
+        def place(t, guard):
+            holder = torch.full((t.numel() + misalign + 16,), 7.0, dtype=dtype, device='cuda')
+            holder[misalign:misalign + t.numel()].copy_(t)
+            guard.append((holder, t.numel()))
+            return holder[misalign:misalign + t.numel()]
+
+        for _ in range(2):                             # a second launch: counters and flags go on
+            guard = []
+            ins = {r: place(host[r], guard) for r in range(algo.ngpus)}
+            outs = {} if algo.inplace else {r: place(torch.zeros(algo.gpus[r].o_chunks * chunk, dtype=dtype), guard) for r in range(algo.ngpus)}
+            got = ex.run(plan, ins, outs, direct=direct)
+            ex.check()
+            for r in range(algo.ngpus):
+                n = min(got[r].numel(), want[r].numel())
+                assert torch.equal(got[r].cpu()[:n].view(torch.uint8), want[r][:n].view(torch.uint8)), f'rank {r} differs'
+            for holder, n in guard:                    # nothing beside the buffers was written
+                assert torch.all(holder[:misalign] == 7) and torch.all(holder[misalign + n:] == 7)
+        geometry = next(iter(plan.geometry.values()))
+        assert geometry[1] >= streams
+        plan.close()
+    finally:
+        comm.close()
+
+
+@pytest.mark.parametrize('name', ['ring', 'two_shot', 'alltoall', 'reduce_scatter'])
+@pytest.mark.parametrize('chunk', [65536, 65536 + 8, 70000])
+def test_several_slices_per_cta(name, chunk, monkeypatch):
+    # tiles of 2 KB: two CTAs' worth of slices with several tiles each, the last one short
+    _check(_algo(name, 4, 'Simple'), chunk, torch.bfloat16, tile=2048, monkeypatch=monkeypatch, streams=1 if name == 'alltoall' else 4)
+
+
+@pytest.mark.parametrize('name', ['ring', 'two_shot', 'allgather', 'reduce_scatter', 'alltoall'])
+@pytest.mark.parametrize('dtype,chunk,misalign', [(torch.float16, 1, 0), (torch.float16, 7, 1), (torch.bfloat16, 9, 5), (torch.float32, 3, 1),
+                                                  (torch.float16, 3071, 0), (torch.bfloat16, 12345, 7), (torch.float32, 4097, 3),
+                                                  (torch.float16, 50001, 2)])
+@pytest.mark.parametrize('direct', [True, False])
+def test_every_alignment(name, dtype, chunk, misalign, direct):
+    _check(_algo(name, 3, 'Simple'), chunk, dtype, misalign, direct=direct)
+
+
+@pytest.mark.parametrize('protocol', ['Simple', 'LL', 'LL128'])
+@pytest.mark.parametrize('name,ranks', [('one_shot', 2), ('one_shot', 9), ('one_shot', 12), ('two_shot', 8)])
+def test_folded_reduces(name, ranks, protocol):
+    # 9 and 12 ranks: eight and eleven adds, a whole batch and more than one
+    _check(_algo(name, ranks, protocol), 2056, torch.bfloat16)
+
+
+def test_small_fifos_and_flag_protocols():
+    for protocol in ('LL', 'LL128'):
+        _check(_algo('ring', 4, protocol), 40008, torch.float16, fifo_bytes=1 << 20)

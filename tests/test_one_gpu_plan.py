@@ -4,8 +4,10 @@ import torch
 
 from msccl.interp import input_chunks_of, run_algorithm
 from msccl.language import MSCCLProgram, ThreadblockPolicy
-from msccl.language.collectives import AllReduce
+from msccl.language.collectives import AllGather, AllReduce, AllToAll, ReduceScatter
+from msccl.programs.allgather import allgather_direct, allgather_ring, reduce_scatter_direct
 from msccl.programs.allreduce import allreduce_allpairs, allreduce_one_shot, allreduce_ring, allreduce_two_shot
+from msccl.programs.alltoall import alltoall_direct
 from msccl.runtime import plan as P
 from msccl.topologies import fully_connected
 from msccl.xml import load_xml
@@ -45,6 +47,27 @@ def test_folded_chains_round_like_the_program(name, ranks, instances):
     want = run_algorithm(algo, host, 24, dtype=torch.bfloat16)
     got = run_algorithm(folded, host, 24, dtype=torch.bfloat16)
     assert all(torch.equal(w.view(torch.int16), g.view(torch.int16)) for w, g in zip(want, got))
+
+
+@pytest.mark.parametrize('coll,body,moves', [
+    (lambda n: AllToAll(n, 1, False), alltoall_direct, True), (lambda n: AllGather(n, 1, False), allgather_direct, True),
+    (lambda n: AllGather(n, 1, False), lambda n: allgather_ring(n, 2), None), (lambda n: ReduceScatter(n, 1, False), reduce_scatter_direct, None)])
+@pytest.mark.parametrize('ranks,instances', [(2, 1), (4, 1), (8, 2)])
+def test_copies_that_move_to_threadblocks_of_their_own(coll, body, moves, ranks, instances):
+    prog = MSCCLProgram('p', fully_connected(ranks), coll(ranks), instances)
+    with prog:
+        body(ranks)
+    algo = load_xml(prog.generate_xml())
+    split = P.split_copies(algo, 256)
+    assert validate(split) == [] and split.num_steps() == algo.num_steps()
+    assert P.split_copies(algo, algo.num_threadblocks()) is algo
+    if moves and ranks > 2:
+        assert split.num_threadblocks() == algo.num_threadblocks() + ranks * instances
+        assert max(sum(st.type in ('s', 'cpy') for st in tb.steps) for g in split.gpus for tb in g.tbs) == 1
+    gen = torch.Generator().manual_seed(4)
+    host = [torch.randn(input_chunks_of(algo, r) * 8, generator=gen) for r in range(ranks)]
+    want, got = run_algorithm(algo, host, 8), run_algorithm(split, host, 8)
+    assert all(torch.equal(w, g) for w, g in zip(want, got))
 
 
 @pytest.mark.parametrize('chunk,esize', [(1, 2), (7, 4), (8, 2), (333333, 2), (4096, 4), (1 << 22, 2), (5 * (1 << 20) + 8, 4)])
