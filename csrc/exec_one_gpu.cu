@@ -697,6 +697,7 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
               out1 = direct_send ? static_cast<char*>(a.ranks[send_peer].buf[st.rbuf]) + (static_cast<long long>(st.roff) * C + tile_off) * esize
                                  : send_fifo + (sseq % kFifoSlots) * slot_bytes;
             int kind = JOB_MOVE;
+            long long tile_byte = 0;                             // where this threadblock's part of the tile starts
             const char *in = nullptr, *add = nullptr;
             char* out0 = nullptr;
             long long in_step = chunk_step;
@@ -721,19 +722,30 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
                 break;
               default: kind = JOB_NONE; break;
             }
-            int nsrc = 0;
+            int nsrc = 0, n = V;
+            if (st.part != 0) {
+              // one part of every chunk, in whole accesses; the other parts are other threadblocks'
+              const int parts = st.part >> 4, part = st.part & 15;
+              const int first = static_cast<int>(static_cast<long long>(V) * part / parts);
+              n = static_cast<int>(static_cast<long long>(V) * (part + 1) / parts) - first;
+              tile_byte = static_cast<long long>(first) * W;
+              in += tile_byte;
+              out0 += tile_byte;
+              if (add != nullptr) add += tile_byte;
+              if (n == 0) kind = JOB_NONE;
+            }
             if (kind == JOB_BATCH) {
               for (int k = 0; k < nb; ++k) {
                 const DevStep& sk = sp[s + g + k];
                 if (sk.type == ST_RE && nsrc < kMaxBatch)
-                  job.src[nsrc++] = static_cast<char*>(me.buf[sk.srcbuf]) + (static_cast<long long>(sk.srcoff) * C + tile_off) * esize;
+                  job.src[nsrc++] = static_cast<char*>(me.buf[sk.srcbuf]) + (static_cast<long long>(sk.srcoff) * C + tile_off) * esize + tile_byte;
               }
             }
             job.in = in; job.add = add; job.out0 = out0; job.out1 = out1;
             job.in_step = in_step; job.add_step = chunk_step; job.out0_step = chunk_step;
             job.out1_step = direct_send ? chunk_step : fifo_chunk;
             job.src_step = chunk_step;
-            job.kind = kind; job.cnt = st.cnt; job.n = V; job.nsrc = nsrc;
+            job.kind = kind; job.cnt = st.cnt; job.n = n; job.nsrc = nsrc;
             if (PROTO != PROTO_SIMPLE) {
               job.flag_in = flag_epoch | (static_cast<unsigned int>((rseq - rseq0) % 4095ull) + 1u);
               job.flag_out = flag_epoch | (static_cast<unsigned int>((sseq - sseq0) % 4095ull) + 1u);

@@ -83,7 +83,8 @@ struct alignas(16) DevStep {    // 32 bytes, copied as two 16-byte vectors
   uint8_t rbuf;                 // SF_DIRECT_SEND: buffer of the matching receive on the peer
   uint8_t batch;                // >1: this and the next batch-1 steps (`re` into this step's dst, or `nop`) run as one
                                 //     multi-input add with one store
-  uint8_t pad0;
+  uint8_t part;                 // ST_RE: parts << 4 | part of every chunk that this threadblock adds; 0: all of it
+                                //     (exec_one_gpu.cu only)
   int32_t roff;                 // SF_DIRECT_SEND: chunk offset of the matching receive on the peer
   uint16_t opens_after;         // receives of this threadblock whose slots may be opened once this step has completed
   uint16_t opens_before;        // receives opened by this (receive) step itself, after its dependency wait

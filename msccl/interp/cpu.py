@@ -171,7 +171,12 @@ class Interpreter:
             src = self.view(rank, st.srcbuf, st.srcoff, st.cnt)
             dst = self.view(rank, st.dstbuf, st.dstoff, st.cnt)
             self._touch(key, rank, st.srcbuf, st.srcoff, st.cnt, False, what)
-            self._touch(key, rank, st.dstbuf, st.dstoff, st.cnt, True, what)
+            if st.part == 0:                       # the parts of one step do not overlap
+                self._touch(key, rank, st.dstbuf, st.dstoff, st.cnt, True, what)
+            if st.parts > 1:
+                src, dst = src.view(st.cnt, -1), dst.view(st.cnt, -1)
+                cut = [src.shape[1] * k // st.parts for k in (st.part, st.part + 1)]
+                src, dst = src[:, cut[0]:cut[1]], dst[:, cut[0]:cut[1]]
             if t == 'cpy':
                 dst.copy_(src)
             else:

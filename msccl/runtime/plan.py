@@ -203,7 +203,7 @@ def _batches(tb):
             if nx.type == 'nop':
                 j += 1
                 continue
-            same_dst = nx.type == 're' and (nx.dstbuf, nx.dstoff, nx.cnt) == (st.dstbuf, st.dstoff, st.cnt)
+            same_dst = nx.type == 're' and (nx.dstbuf, nx.dstoff, nx.cnt, nx.part, nx.parts) == (st.dstbuf, st.dstoff, st.cnt, st.part, st.parts)
             # a source that overlaps the destination must see the partial sum of the steps before it: not batched
             overlaps = nx.type == 're' and nx.srcbuf == st.dstbuf and nx.srcoff < st.dstoff + st.cnt and st.dstoff < nx.srcoff + nx.cnt
             if not same_dst or overlaps:
@@ -321,8 +321,10 @@ def _find_chain(algo, gpu, waiters, limit):
 
 def fold_reduce_chains(algo: AlgoIR) -> AlgoIR:
     """The program with chains of local reduces that pass a slot from threadblock to threadblock (n - 1 hops of store,
-    fence, flag and poll in the one-shot and two-shot all-reduce) replaced by one multi-input add at the end of the chain
-    - same operands, same order, same roundings.  The input is not modified."""
+    fence, flag and poll in the one-shot and two-shot all-reduce) replaced by one multi-input add - same operands, same
+    order, same roundings - of which every threadblock of the chain does its part of each chunk.  Whoever waited for the
+    end of the chain waits for all parts (two-shot all-reduce of 64 MB over 8 ranks: 848 us with the whole add in the last
+    threadblock, 505 in parts).  The input is not modified."""
     gpus, changed = [], False
     for g in algo.gpus:
         gpu = replace(g, tbs=[replace(tb, steps=[replace(st) for st in tb.steps]) for tb in g.tbs])
@@ -335,48 +337,70 @@ def fold_reduce_chains(algo: AlgoIR) -> AlgoIR:
             if chain is None:
                 break
             changed = True
-            last_t, last_i = chain[-1]
-            removed = {t: set() for t, _ in chain}
-            head, adds = {}, []          # tb -> latest step that must be done before the first add; the adds in chain order
+            end = chain[-1]
+            removed = set(chain)
+            head, pred = {}, {}          # tb -> latest step that must be done before the first add / that fills a source
             for k, (t, i) in enumerate(chain):
                 steps = gpu.tbs[t].steps
-                removed[t].add(i)
                 deps = [steps[i]] if k == 0 else []
                 j = i - 1
                 while j >= 0 and steps[j].type == 'nop' and waiters[(t, j)] == 0 and not steps[j].hasdep:
                     deps.append(steps[j])
-                    removed[t].add(j)
+                    removed.add((t, j))
                     j -= 1
                 for st in deps:
-                    if st.depid >= 0 and st.depid != last_t:
+                    if st.depid >= 0:
                         head[st.depid] = max(head.get(st.depid, -1), st.deps)
-                add = replace(steps[i], depid=-1, deps=-1, hasdep=False)
-                if t != last_t and j >= 0:                  # what came before the link fills its source
+                if j >= 0:
                     steps[j].hasdep = True
-                    add.depid, add.deps = t, j
-                adds.append(add)
-            for add in adds:
-                if add.depid in head:                       # one wait per threadblock, the later of the two
-                    head[add.depid] = max(head[add.depid], add.deps)
-                    add.depid = add.deps = -1
-            hasdep = gpu.tbs[last_t].steps[last_i].hasdep
-            group = [replace(adds[0], type='nop', srcbuf='i', srcoff=-1, dstbuf='o', dstoff=-1, cnt=0, depid=d, deps=s)
-                     for d, s in sorted(head.items())] + adds
-            group[-1].hasdep = hasdep
+                    pred[t] = j
+            links = [gpu.tbs[t].steps[i] for t, i in chain]
+
+            def nop(dep):
+                return replace(links[0], type='nop', srcbuf='i', srcoff=-1, dstbuf='o', dstoff=-1, cnt=0, depid=dep[0], deps=dep[1],
+                               hasdep=False)
+
+            groups = {}
+            for k, (t, i) in enumerate(chain):
+                first = {d: s for d, s in head.items() if d != t}
+                adds = []
+                for (source, _), st in zip(chain, links):
+                    add = replace(st, depid=-1, deps=-1, hasdep=False, part=k, parts=len(chain))
+                    if source != t and source in pred:
+                        if source in first:             # one wait per threadblock, the later of the two
+                            first[source] = max(first[source], pred[source])
+                        else:
+                            add.depid, add.deps = source, pred[source]
+                    adds.append(add)
+                adds[-1].hasdep = True
+                groups[(t, i)] = [nop(dep) for dep in sorted(first.items())] + adds
+            # whoever waited for the end, or came behind it, waits for every part (its own threadblock's is behind it anyway)
+            in_front = {}
+            for t, tb in enumerate(gpu.tbs):
+                for i, st in enumerate(tb.steps):
+                    if (t, i) in removed:
+                        continue
+                    parts = [c for c in chain if c[0] != t]
+                    if (st.depid, st.deps) == end:
+                        in_front[(t, i)] = [nop(dep) for dep in parts[:-1]]
+                        st.depid, st.deps = parts[-1]
+                    elif (t, i) == (end[0], end[1] + 1):
+                        in_front[(t, i)] = [nop(dep) for dep in parts]
             renumber = {}
-            for t in removed:
+            for t, tb in enumerate(gpu.tbs):
                 fresh = []
-                for i, st in enumerate(gpu.tbs[t].steps):
-                    if (t, i) == (last_t, last_i):
-                        fresh.extend(group)
-                    elif i not in removed[t]:
+                for i, st in enumerate(tb.steps):
+                    if (t, i) in groups:
+                        fresh.extend(groups[(t, i)])
+                    elif (t, i) not in removed:
+                        fresh.extend(in_front.get((t, i), []))
                         fresh.append(st)
                     renumber[(t, i)] = len(fresh) - 1
-                gpu.tbs[t].steps = fresh
+                tb.steps = fresh
             for tb in gpu.tbs:
                 for i, st in enumerate(tb.steps):
                     st.s = i
-                    if (st.depid, st.deps) in renumber:
+                    if st.depid >= 0:
                         st.deps = renumber[(st.depid, st.deps)]
     return replace(algo, gpus=gpus) if changed else algo
 
@@ -470,7 +494,8 @@ def compile_plan(algo: AlgoIR, local_ranks, slot_bytes: int, check=True, direct=
                 if nb:
                     plan.batched_steps += sum(1 for k in range(si, si + nb) if tb.steps[k].type == 're')
                 packed.append(_STEP.pack(STEP_CODES[st.type], BUF_CODES[sbuf], BUF_CODES[dbuf], int(st.hasdep),
-                                         st.depid, st.deps, soff, doff, cnt, flags, rbuf, nb, 0, roff,
+                                         st.depid, st.deps, soff, doff, cnt, flags, rbuf, nb,
+                                         st.parts << 4 | st.part if st.parts > 1 else 0, roff,
                                          opens_after.get(si, 0), opens_before.get(si, 0)))
             if nrecv > 0 and recv_mask and at_start == nrecv:
                 plan.eager_tbs += 1

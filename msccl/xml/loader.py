@@ -38,6 +38,8 @@ class StepIR:
     depid: int
     deps: int
     hasdep: bool
+    part: int = 0           # a plan may run one part of `parts` of every chunk here (not part of the XML)
+    parts: int = 1
 
     def is_send(self):
         return self.type in SEND_TYPES
