@@ -8,7 +8,9 @@
 // order of K, whatever order the pairs finish in; no workspace, no atomics.
 //
 // S = 4 when all tiles fit into clusters of eight at once, else S = 2 when they fit into clusters of four; with more tiles
-// than that the persistent kernel already fills half of the GPU.
+// than that the persistent kernel already fills half of the GPU.  Shorter sums than 16 k blocks do not pay for the exchange.
+// Persistent kernel / this one, device time in us: 14 tiles K = 1024 13.0 / 12.0, 4096 26.6 / 15.8, 8192 44.4 / 20.8 (S = 4);
+// 32 tiles K = 512 9.0 / 9.9, 1024 11.5 / 11.2, 4096 25.0 / 19.0, 8192 43.4 / 29.8 (S = 2).
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -256,8 +258,9 @@ cudaError_t launch_split(const CUtensorMap& map_a, const CUtensorMap& map_b, __n
 // How many ways K is split for this shape: 4, 2, or 1 (the persistent kernel).
 int splitk_ways(int M, int N, int K, int epilogue) {
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * (N / PBN), k_blocks = K / BK;
-  if (k_blocks >= 16 && tiles <= (epilogue ? max_clusters<1, 4>() : max_clusters<0, 4>())) return 4;
-  if (k_blocks >= 8 && tiles <= (epilogue ? max_clusters<1, 2>() : max_clusters<0, 2>())) return 2;
+  if (k_blocks < 16) return 1;
+  if (tiles <= (epilogue ? max_clusters<1, 4>() : max_clusters<0, 4>())) return 4;
+  if (tiles <= (epilogue ? max_clusters<1, 2>() : max_clusters<0, 2>())) return 2;
   return 1;
 }
 
