@@ -23,13 +23,15 @@ Execution model (the contract the native executor implements as well):
 Scheduling is cooperative and deterministic; if no threadblock can advance the interpreter
 raises ``DeadlockError`` naming the blocked steps.  With ``race_check=True`` every access to a
 chunk is checked against earlier conflicting accesses using vector clocks over program order,
-dependency edges and message edges; an unordered pair raises ``RaceError``.
+dependency edges and message edges; an unordered pair raises ``RaceError``.  A step that does one part of its chunks
+(``StepIR.part``) touches that part only.
 
 Arithmetic: element type is the tensor dtype; sums of bf16/fp16 are computed in fp32 and
 rounded once per addition (torch CPU semantics), which is what the CUDA kernels do as well,
 so results can be compared bit for bit.
 """
 from collections import defaultdict, deque
+from fractions import Fraction
 
 import torch
 
@@ -88,8 +90,13 @@ class Interpreter:
         # race checking state
         self.clock = {key: _Clock() for key in self.pc}
         self.done_clock = {}                 # (rank, tb, step) -> clock snapshot after the step
-        self.last_write = {}                 # (rank, buf, chunk) -> (tb key, time, description)
+        self.last_write = {}                 # (rank, buf, chunk, cell) -> (tb key, time, description)
         self.reads_since = defaultdict(list)
+        # (part, parts) -> the cells of a chunk that such a step touches; a cell lies between two places where some step of the
+        # program cuts its chunks
+        sizes = {1} | {st.parts for g in algo.gpus for tb in g.tbs for st in tb.steps}
+        cuts = sorted({Fraction(k, n) for n in sizes for k in range(n + 1)})
+        self.cells = {(k, n): range(cuts.index(Fraction(k, n)), cuts.index(Fraction(k + 1, n))) for n in sizes for k in range(n)}
         # cross-rank barriers
         self.bar_passed = defaultdict(int)   # tb key -> barriers passed
         self.bar_arrived = defaultdict(dict)  # (channel, index) -> {rank: clock snapshot}
@@ -121,13 +128,13 @@ class Interpreter:
         return self.buffers[rank]['o']
 
     # ------------------------------------------------------------ race checks
-    def _touch(self, key, rank, buf, off, cnt, write, what):
+    def _touch(self, key, rank, buf, off, cnt, write, what, part=0, parts=1):
         if not self.race_check:
             return
         clock = self.clock[key]
         rbuf, roff = self.algo.resolve(rank, buf, off)
-        for i in range(roff, roff + cnt):
-            slot = (rank, rbuf, i)
+        for i, cell in ((i, cell) for i in range(roff, roff + cnt) for cell in self.cells[part, parts]):
+            slot = (rank, rbuf, i, cell)
             prev = self.last_write.get(slot)
             if prev is not None and prev[0] != key and not clock.covers(prev[0], prev[1]):
                 raise RaceError(f'{what} on gpu {rank} {rbuf}[{i}] is not ordered after the write by {prev[2]}')
@@ -170,9 +177,8 @@ class Interpreter:
         elif t in ('cpy', 're'):
             src = self.view(rank, st.srcbuf, st.srcoff, st.cnt)
             dst = self.view(rank, st.dstbuf, st.dstoff, st.cnt)
-            self._touch(key, rank, st.srcbuf, st.srcoff, st.cnt, False, what)
-            if st.part == 0:                       # the parts of one step do not overlap
-                self._touch(key, rank, st.dstbuf, st.dstoff, st.cnt, True, what)
+            self._touch(key, rank, st.srcbuf, st.srcoff, st.cnt, False, what, st.part, st.parts)
+            self._touch(key, rank, st.dstbuf, st.dstoff, st.cnt, True, what, st.part, st.parts)
             if st.parts > 1:
                 src, dst = src.view(st.cnt, -1), dst.view(st.cnt, -1)
                 cut = [src.shape[1] * k // st.parts for k in (st.part, st.part + 1)]

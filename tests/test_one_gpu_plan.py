@@ -1,8 +1,10 @@
 """Host side of the one-GPU interpreter: folded reduce chains against the unfolded program, and its launch geometry."""
+from dataclasses import replace
+
 import pytest
 import torch
 
-from msccl.interp import input_chunks_of, run_algorithm
+from msccl.interp import RaceError, input_chunks_of, run_algorithm
 from msccl.language import MSCCLProgram, ThreadblockPolicy
 from msccl.language.collectives import AllGather, AllReduce, AllToAll, ReduceScatter
 from msccl.programs.allgather import allgather_direct, allgather_ring, reduce_scatter_direct
@@ -68,6 +70,47 @@ def test_copies_that_move_to_threadblocks_of_their_own(coll, body, moves, ranks,
     host = [torch.randn(input_chunks_of(algo, r) * 8, generator=gen) for r in range(ranks)]
     want, got = run_algorithm(algo, host, 8), run_algorithm(split, host, 8)
     assert all(torch.equal(w, g) for w, g in zip(want, got))
+
+
+def _copy(algo):
+    return replace(algo, gpus=[replace(g, tbs=[replace(tb, steps=[replace(st) for st in tb.steps]) for tb in g.tbs]) for g in algo.gpus])
+
+
+def _race_check(algo, chunk=24):
+    host = [torch.ones(input_chunks_of(algo, r) * chunk) for r in range(algo.ngpus)]
+    run_algorithm(algo, host, chunk, race_check=True)
+
+
+@pytest.mark.parametrize('name,ranks,instances', [('one_shot', 3, 2), ('one_shot', 8, 1), ('two_shot', 4, 1), ('two_shot', 8, 2),
+                                                  ('one_shot', 9, 1), ('one_shot', 12, 1), ('ring', 4, 2), ('allpairs', 4, 1)])
+def test_rewritten_programs_are_free_of_races(name, ranks, instances):
+    folded = P.fold_reduce_chains(_program(name, ranks, instances))
+    _race_check(folded)
+    _race_check(P.split_copies(folded, 1 << 20))
+
+
+@pytest.mark.parametrize('name,ranks', [('two_shot', 4), ('two_shot', 8), ('one_shot', 3), ('one_shot', 12)])
+def test_a_wait_that_is_dropped_from_a_folded_program_is_a_race(name, ranks):
+    """Every wait for one part of an add (and for what fills its sources) is needed, whichever part it is.  With 12 ranks a chain of
+    eight adds follows one of three: a part of the second waits for all three and overlaps with one or two of them."""
+    folded = P.fold_reduce_chains(_program(name, ranks))
+    dropped = races = parts_after_the_first = 0
+    for t, tb in enumerate(folded.gpus[0].tbs):
+        for i, st in enumerate(tb.steps):
+            if st.depid < 0:
+                continue
+            awaited = folded.gpus[0].tbs[st.depid].steps[st.deps]
+            less = _copy(folded)
+            less.gpus[0].tbs[t].steps[i].depid = less.gpus[0].tbs[t].steps[i].deps = -1
+            dropped += 1
+            try:
+                _race_check(less)
+            except RaceError:
+                races += 1
+                parts_after_the_first += awaited.type == 're' and awaited.part > 0
+    # 8 x 3 pairs of parts, of which 8 + 3 - gcd(8, 3) overlap
+    assert races == dropped - ((8 * 3 - 10) if ranks == 12 else 0) > 0
+    assert parts_after_the_first > 0 or (name, ranks) == ('one_shot', 3)
 
 
 @pytest.mark.parametrize('chunk,esize', [(1, 2), (7, 4), (8, 2), (333333, 2), (4096, 4), (1 << 22, 2), (5 * (1 << 20) + 8, 4)])
