@@ -21,9 +21,10 @@ Besides the translation, three analyses run here:
 import struct
 from collections import Counter
 from dataclasses import dataclass, field, replace
+from itertools import count
 from typing import Dict, List
 
-from msccl.xml.loader import AlgoIR
+from msccl.xml.loader import AlgoIR, StepIR
 from msccl.xml.validator import validate
 
 STEP_CODES = {'nop': 0, 's': 1, 'r': 2, 'rcs': 3, 'rrs': 4, 'rrc': 5, 'rrcs': 6, 'cpy': 7, 're': 8}
@@ -219,6 +220,12 @@ def _batches(tb):
     return out
 
 
+def _dependencies_exist(gpu):
+    """False: the validator will report the program, which is left as it is."""
+    return all(st.depid < 0 or (st.depid < len(gpu.tbs) and 0 <= st.deps < len(gpu.tbs[st.depid].steps))
+               for tb in gpu.tbs for st in tb.steps)
+
+
 def split_copies(algo: AlgoIR, most_tbs: int) -> AlgoIR:
     """The program with local copies that nothing depends on in threadblocks of their own.
 
@@ -231,7 +238,7 @@ def split_copies(algo: AlgoIR, most_tbs: int) -> AlgoIR:
     for g in algo.gpus:
         gpu = replace(g, tbs=[replace(tb, steps=[replace(st) for st in tb.steps]) for tb in g.tbs])
         gpus.append(gpu)
-        if any(tb.id != i for i, tb in enumerate(gpu.tbs)):
+        if any(tb.id != i for i, tb in enumerate(gpu.tbs)) or not _dependencies_exist(gpu):
             continue
         steps = [(t, i, st) for t, tb in enumerate(gpu.tbs) for i, st in enumerate(tb.steps)]
         waited = {(st.depid, st.deps) for _, _, st in steps if st.depid >= 0}
@@ -271,52 +278,129 @@ def _overlap(o1, c1, o2, c2):
     return o1 < o2 + c2 and o2 < o1 + c1
 
 
-def _find_chain(algo, gpu, waiters, limit):
-    """A chain of ``re`` steps into one slot, each in another threadblock and waiting for the one before, that may run as
-    one multi-input add at the place of the last one.  Returns ``[(tb, step), ...]`` or None.
+_NOP = StepIR(0, 'nop', 'i', -1, 'o', -1, 0, -1, -1, False)
+
+
+class _Node:
+    """A step while its program is rewritten: its neighbours in the threadblock ``tb``, the step it waits for, the steps that wait
+    for it, and a ``key`` that orders the steps of a threadblock."""
+    __slots__ = ('st', 'tb', 'key', 'prev', 'next', 'dep', 'waiters')
+
+    def __init__(self, st, tb, key):
+        self.st, self.tb, self.key = st, tb, key
+        self.prev = self.next = self.dep = None
+        self.waiters = set()
+
+    def wait_for(self, node):
+        if self.dep is not None:
+            self.dep.waiters.discard(self)
+        self.dep = node
+        if node is not None:
+            node.waiters.add(self)
+
+    def put_in_front(self, fresh):
+        for node in fresh:
+            node.prev, node.next = self.prev, self
+            self.prev.next = self.prev = node
+
+    def remove(self):
+        self.prev.next = self.next
+        self.next.prev = self.prev
+        self.wait_for(None)
+
+
+def _linked(gpu):
+    """The steps of every threadblock as linked ``_Node``s: the end mark in front of each (another one is behind)."""
+    fronts, rows = [], [[_Node(st, t, (i, 0, 0)) for i, st in enumerate(tb.steps)] for t, tb in enumerate(gpu.tbs)]
+    for t, row in enumerate(rows):
+        front, back = (_Node(replace(_NOP, type='end'), t, (i, 0, 0)) for i in (-1, len(row)))
+        front.next, back.prev = back, front
+        back.put_in_front(row)
+        fronts.append(front)
+        for node in row:
+            if node.st.depid >= 0:
+                node.wait_for(rows[node.st.depid][node.st.deps])
+    return fronts
+
+
+def _chain_to(end, slot, limit):
+    """The chain of ``re`` steps into one slot, each in another threadblock and waiting for the one before, that ends with
+    ``end`` and may run as one multi-input add at its place: ``[node, ...]``, or None.
 
     A link may be taken out of its threadblock when nobody but the next link waits for it and whatever follows it in
     its threadblock already waits for the end of the chain: then everything that was ordered after a link is ordered
     after the end, and everything that came before a link is waited for by the end."""
-    def slot(st, src):
-        return algo.resolve(gpu.id, st.srcbuf, st.srcoff) if src else algo.resolve(gpu.id, st.dstbuf, st.dstoff)
+    def alone(node):                                            # not one of a run of adds in its threadblock
+        return node.prev.st.type != 're'
 
-    for t, tb in enumerate(gpu.tbs):
-        for i, st in enumerate(tb.steps):
-            if st.type != 're' or (i + 1 < len(tb.steps) and tb.steps[i + 1].type == 're'):
-                continue
-            if any(x.type == 're' and x.depid == t and x.deps == i and slot(x, False) == slot(st, False) and
-                   not (j + 1 < len(other.steps) and other.steps[j + 1].type == 're')
-                   for o, other in enumerate(gpu.tbs) if o != t for j, x in enumerate(other.steps)):
-                continue                                    # not the end of its chain
-            chain = [(t, i)]
-            while len(chain) < limit:
-                ct, ci = chain[0]
-                cur = gpu.tbs[ct].steps[ci]
-                if ci > 0 and gpu.tbs[ct].steps[ci - 1].type == 're':
-                    break
-                if not 0 <= cur.depid < len(gpu.tbs) or cur.depid in [x for x, _ in chain]:
-                    break
-                prev_tb = gpu.tbs[cur.depid]
-                if not 0 <= cur.deps < len(prev_tb.steps):
-                    break
-                prev = prev_tb.steps[cur.deps]
-                if (prev.type != 're' or slot(prev, False) != slot(st, False) or prev.cnt != st.cnt or
-                        waiters[(cur.depid, cur.deps)] != 1 or
-                        (cur.deps > 0 and prev_tb.steps[cur.deps - 1].type == 're')):
-                    break
-                if cur.deps + 1 < len(prev_tb.steps):
-                    behind = prev_tb.steps[cur.deps + 1]
-                    if behind.depid != t or behind.deps < i:
-                        break
-                chain.insert(0, (cur.depid, cur.deps))
-            dst = slot(st, False)
-            srcs = [slot(gpu.tbs[ct].steps[ci], True) for ct, ci in chain]
-            if any(b == dst[0] and _overlap(o, st.cnt, dst[1], st.cnt) for b, o in srcs):
-                continue
-            if len(chain) > 1:
-                return chain
-    return None
+    dst = slot(end.st, False)
+    if end.st.type != 're' or end.next.st.type == 're':
+        return None
+    if any(x.st.type == 're' and x.tb != end.tb and slot(x.st, False) == dst and x.next.st.type != 're' for x in end.waiters):
+        return None                                             # not the end of its chain
+    chain = [end]
+    while len(chain) < limit and alone(chain[0]):
+        link = chain[0].dep
+        if (link is None or any(link.tb == node.tb for node in chain) or link.st.type != 're' or slot(link.st, False) != dst or
+                link.st.cnt != end.st.cnt or len(link.waiters) != 1 or not alone(link)):
+            break
+        behind = link.next
+        if behind.st.type != 'end' and (behind.dep is None or behind.dep.tb != end.tb or behind.dep.key < end.key):
+            break
+        chain.insert(0, link)
+    srcs = [slot(node.st, True) for node in chain]
+    if len(chain) < 2 or any(b == dst[0] and _overlap(o, end.st.cnt, dst[1], end.st.cnt) for b, o in srcs):
+        return None
+    return chain
+
+
+def _fold(chain, fresh_key):
+    """Replace ``chain`` by one multi-input add of which each of its threadblocks does a part."""
+    end = chain[-1]
+    head, pred = {}, {}              # tb -> latest step that must be done before the first add / step that fills a source
+    for k, link in enumerate(chain):
+        waits = [link.dep] if k == 0 else []
+        while link.prev.st.type == 'nop' and not link.prev.waiters and not link.prev.st.hasdep:
+            waits.append(link.prev.dep)
+            link.prev.remove()
+        for dep in waits:
+            if dep is not None and (dep.tb not in head or head[dep.tb].key < dep.key):
+                head[dep.tb] = dep
+        if link.prev.st.type != 'end':
+            link.prev.st.hasdep = True
+            pred[link.tb] = link.prev
+
+    def nop(in_front_of, dep):
+        node = _Node(replace(_NOP), in_front_of.tb, (in_front_of.key[0], in_front_of.key[1] - 1, fresh_key()))
+        node.wait_for(dep)
+        return node
+
+    groups = []
+    for k, link in enumerate(chain):
+        first = {tb: dep for tb, dep in head.items() if tb != link.tb}
+        adds = []
+        for source in chain:
+            add = _Node(replace(source.st, hasdep=False, part=k, parts=len(chain)), link.tb, (link.key[0], link.key[1], fresh_key()))
+            dep = pred.get(source.tb) if source.tb != link.tb else None
+            if dep is not None and source.tb in first:          # one wait per threadblock, the later of the two
+                first[source.tb] = max(first[source.tb], dep, key=lambda node: node.key)
+            else:
+                add.wait_for(dep)
+            adds.append(add)
+        adds[-1].st.hasdep = True
+        groups.append([nop(link, dep) for _, dep in sorted(first.items())] + adds)
+    # whoever waited for the end, or came behind it, waits for every part (its own threadblock's is behind it anyway)
+    last = {link.tb: group[-1] for link, group in zip(chain, groups)}
+    for waiter in sorted(end.waiters, key=lambda node: (node.tb, node.key)):
+        parts = [last[link.tb] for link in chain if link.tb != waiter.tb]
+        waiter.put_in_front([nop(waiter, dep) for dep in parts[:-1]])
+        waiter.wait_for(parts[-1])
+    behind = end.next
+    if behind.st.type != 'end':
+        behind.put_in_front([nop(behind, last[link.tb]) for link in chain[:-1]])
+    for link, group in zip(chain, groups):
+        link.put_in_front(group)
+        link.remove()
 
 
 def fold_reduce_chains(algo: AlgoIR) -> AlgoIR:
@@ -324,84 +408,45 @@ def fold_reduce_chains(algo: AlgoIR) -> AlgoIR:
     fence, flag and poll in the one-shot and two-shot all-reduce) replaced by one multi-input add - same operands, same
     order, same roundings - of which every threadblock of the chain does its part of each chunk.  Whoever waited for the
     end of the chain waits for all parts (two-shot all-reduce of 64 MB over 8 ranks: 848 us with the whole add in the last
-    threadblock, 505 in parts).  The input is not modified."""
+    threadblock, 505 in parts).  The input is not modified; a GPU whose threadblocks would get more steps than the interpreter
+    takes keeps its chains.  The time grows with the number of steps only, which a program may have thousands of."""
     gpus, changed = [], False
     for g in algo.gpus:
+        gpus.append(g)
         gpu = replace(g, tbs=[replace(tb, steps=[replace(st) for st in tb.steps]) for tb in g.tbs])
-        gpus.append(gpu)
-        if any(tb.id != i for i, tb in enumerate(gpu.tbs)):
+        if any(tb.id != i for i, tb in enumerate(gpu.tbs)) or not _dependencies_exist(gpu):
             continue
-        while True:
-            waiters = Counter((st.depid, st.deps) for tb in gpu.tbs for st in tb.steps if st.depid >= 0)
-            chain = _find_chain(algo, gpu, waiters, K_MAX_BATCH)
-            if chain is None:
-                break
-            changed = True
-            end = chain[-1]
-            removed = set(chain)
-            head, pred = {}, {}          # tb -> latest step that must be done before the first add / that fills a source
-            for k, (t, i) in enumerate(chain):
-                steps = gpu.tbs[t].steps
-                deps = [steps[i]] if k == 0 else []
-                j = i - 1
-                while j >= 0 and steps[j].type == 'nop' and waiters[(t, j)] == 0 and not steps[j].hasdep:
-                    deps.append(steps[j])
-                    removed.add((t, j))
-                    j -= 1
-                for st in deps:
-                    if st.depid >= 0:
-                        head[st.depid] = max(head.get(st.depid, -1), st.deps)
-                if j >= 0:
-                    steps[j].hasdep = True
-                    pred[t] = j
-            links = [gpu.tbs[t].steps[i] for t, i in chain]
+        fronts = _linked(gpu)
 
-            def nop(dep):
-                return replace(links[0], type='nop', srcbuf='i', srcoff=-1, dstbuf='o', dstoff=-1, cnt=0, depid=dep[0], deps=dep[1],
-                               hasdep=False)
+        def slot(st, src):
+            return algo.resolve(g.id, st.srcbuf, st.srcoff) if src else algo.resolve(g.id, st.dstbuf, st.dstoff)
 
-            groups = {}
-            for k, (t, i) in enumerate(chain):
-                first = {d: s for d, s in head.items() if d != t}
-                adds = []
-                for (source, _), st in zip(chain, links):
-                    add = replace(st, depid=-1, deps=-1, hasdep=False, part=k, parts=len(chain))
-                    if source != t and source in pred:
-                        if source in first:             # one wait per threadblock, the later of the two
-                            first[source] = max(first[source], pred[source])
-                        else:
-                            add.depid, add.deps = source, pred[source]
-                    adds.append(add)
-                adds[-1].hasdep = True
-                groups[(t, i)] = [nop(dep) for dep in sorted(first.items())] + adds
-            # whoever waited for the end, or came behind it, waits for every part (its own threadblock's is behind it anyway)
-            in_front = {}
-            for t, tb in enumerate(gpu.tbs):
-                for i, st in enumerate(tb.steps):
-                    if (t, i) in removed:
-                        continue
-                    parts = [c for c in chain if c[0] != t]
-                    if (st.depid, st.deps) == end:
-                        in_front[(t, i)] = [nop(dep) for dep in parts[:-1]]
-                        st.depid, st.deps = parts[-1]
-                    elif (t, i) == (end[0], end[1] + 1):
-                        in_front[(t, i)] = [nop(dep) for dep in parts]
-            renumber = {}
-            for t, tb in enumerate(gpu.tbs):
-                fresh = []
-                for i, st in enumerate(tb.steps):
-                    if (t, i) in groups:
-                        fresh.extend(groups[(t, i)])
-                    elif (t, i) not in removed:
-                        fresh.extend(in_front.get((t, i), []))
-                        fresh.append(st)
-                    renumber[(t, i)] = len(fresh) - 1
-                tb.steps = fresh
-            for tb in gpu.tbs:
-                for i, st in enumerate(tb.steps):
-                    st.s = i
-                    if st.depid >= 0:
-                        st.deps = renumber[(st.depid, st.deps)]
+        fresh_key, found, more = count(1).__next__, False, True
+        while more:
+            more = False
+            for front in fronts:
+                node = front.next
+                while node.st.type != 'end':
+                    behind = node.next
+                    chain = _chain_to(node, slot, K_MAX_BATCH)
+                    if chain is not None:
+                        _fold(chain, fresh_key)
+                        found = more = True
+                    node = behind
+        if not found:
+            continue
+        for tb, front in zip(gpu.tbs, fronts):
+            tb.steps, node = [], front.next
+            while node.st.type != 'end':
+                node.st.s, node.key = len(tb.steps), len(tb.steps)
+                tb.steps.append(node)
+                node = node.next
+        for tb in gpu.tbs:
+            for node in tb.steps:
+                node.st.depid, node.st.deps = (-1, -1) if node.dep is None else (node.dep.tb, node.dep.key)
+            tb.steps = [node.st for node in tb.steps]
+        if max(len(tb.steps) for tb in gpu.tbs) <= K_MAX_STEPS_PER_TB:
+            gpus[-1], changed = gpu, True
     return replace(algo, gpus=gpus) if changed else algo
 
 

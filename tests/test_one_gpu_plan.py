@@ -1,4 +1,5 @@
 """Host side of the one-GPU interpreter: folded reduce chains against the unfolded program, and its launch geometry."""
+import time
 from dataclasses import replace
 
 import pytest
@@ -49,6 +50,52 @@ def test_folded_chains_round_like_the_program(name, ranks, instances):
     want = run_algorithm(algo, host, 24, dtype=torch.bfloat16)
     got = run_algorithm(folded, host, 24, dtype=torch.bfloat16)
     assert all(torch.equal(w.view(torch.int16), g.view(torch.int16)) for w, g in zip(want, got))
+
+
+def _rounds(ranks, rounds):
+    """The one-shot all-reduce ``rounds`` times: the sends of a round wait for the sum of the one before."""
+    algo = _copy(_program('one_shot', ranks))
+    for gpu in algo.gpus:
+        once = [tb.steps for tb in gpu.tbs]
+        waited = {(st.depid, st.deps) for steps in once for st in steps}
+        end_tb, end = next((t, i) for t, steps in enumerate(once) for i, st in enumerate(steps)
+                           if st.type == 're' and (t, i) not in waited)
+        once[end_tb][end].hasdep = True
+        for t, tb in enumerate(gpu.tbs):
+            tb.steps = []
+            for k in range(rounds):
+                for st in once[t]:
+                    st = replace(st, s=len(tb.steps), deps=st.deps + k * len(once[st.depid]) if st.depid >= 0 else -1)
+                    if k and st.type == 's' and t != end_tb:
+                        st.depid, st.deps = end_tb, (k - 1) * len(once[end_tb]) + end
+                    tb.steps.append(st)
+    return algo
+
+
+def test_long_programs_fold_in_time():
+    # 2600 steps per GPU, 100 chains: a search that starts again behind every chain takes minutes, one pass a second
+    algo = _rounds(8, 100)
+    assert validate(algo) == []
+    start = time.perf_counter()
+    folded = P.fold_reduce_chains(algo)
+    assert time.perf_counter() - start < 20
+    assert validate(folded) == [] and sum(st.parts == 7 for tb in folded.gpus[0].tbs for st in tb.steps) == 7 * 7 * 100
+
+
+def test_programs_that_would_get_too_long_stay_as_they_are(monkeypatch):
+    algo = _rounds(4, 10)
+    assert P.fold_reduce_chains(algo) is not algo
+    monkeypatch.setattr(P, 'K_MAX_STEPS_PER_TB', max(len(tb.steps) for tb in algo.gpus[0].tbs))
+    assert P.fold_reduce_chains(algo) is algo
+    P.compile_plan(P.fold_reduce_chains(algo), range(4), 64 << 10)
+
+
+def test_dependencies_on_missing_steps_are_left_to_the_validator():
+    algo = _copy(_program('one_shot', 3))
+    next(st for tb in algo.gpus[0].tbs for st in tb.steps if st.type == 're' and st.depid >= 0).deps = 99
+    algo.gpus[1].tbs[0].steps[-1].depid = 7
+    with pytest.raises(P.PlanError):
+        P.compile_plan(P.split_copies(P.fold_reduce_chains(algo), 64), range(3), 64 << 10)
 
 
 @pytest.mark.parametrize('coll,body,moves', [
