@@ -621,7 +621,8 @@ def one_gpu_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_byte
         raise PlanError('FIFO slot too small for this program')
     if proto == 0 and not (plan.single_hop and direct):
         want = max(per_access, ONE_GPU_TILE_BYTES // plan.max_cnt // elem_size // line * line)
-        want = max(want, -(-slice_elems // (K_MAX_ITERATIONS - 1) // per_access + 1) * per_access)
+        least = -(-slice_elems // (K_MAX_ITERATIONS - 1))                        # fewer would be too many iterations
+        want = max(want, -(-least // per_access) * per_access)
         tile = min(tile, want)
     tile = min(tile, slice_elems)
     if -(-slice_elems // tile) >= K_MAX_ITERATIONS:

@@ -176,3 +176,40 @@ def test_one_gpu_geometry_covers_the_chunk(chunk, esize, proto, max_ctas):
     accesses = tile * esize // width
     fifo = {0: accesses * width, 1: accesses * (32 if width == 16 else 8), 2: -(-2 * accesses // 15) * 128}[proto]
     assert fifo * plan.max_cnt <= slot
+
+
+def _wide(count):
+    """Two ranks, one message of ``count`` chunks, stored by the receiver (``rrc``: never straight into its slot)."""
+    tb = '<tb id="0" send="{}" recv="{}" chan="0"><step s="0" type="{}" srcbuf="i" srcoff="0" dstbuf="i" dstoff="0" cnt="{}" ' \
+         'depid="-1" deps="-1" hasdep="0"/></tb>'
+    gpu = '<gpu id="{}" i_chunks="{}" o_chunks="0" s_chunks="0">{}</gpu>'
+    return load_xml('<algo name="wide" proto="Simple" nchannels="1" nchunksperloop="1" ngpus="2" coll="custom" inplace="1">' +
+                    gpu.format(0, count, tb.format(1, -1, 's', count)) + gpu.format(1, count, tb.format(-1, 0, 'rrc', count)) + '</algo>')
+
+
+@pytest.mark.parametrize('count,chunk,slot_bytes,max_ctas', [(1, 1 << 33, 4 << 20, 592), (1025, 1 << 28, 4 << 20, 2), (1025, 1 << 33, 256 << 20, 592),
+                                                             (2000, 9 * (1 << 20) * 196, 256 << 20, 16), (4097, 1 << 28, 256 << 20, 16)])
+def test_tiles_of_wide_steps_keep_within_the_iteration_limit(count, chunk, slot_bytes, max_ctas):
+    """128 KB over more than a thousand chunks leaves tiles of less than a line: they grow until the iterations fit."""
+    plan = P.compile_plan(_wide(count), range(2), slot_bytes)
+    assert P.tile_geometry(plan, chunk, 2, slot_bytes)[1] < P.K_MAX_ITERATIONS
+    _, _, slice_elems, tile, slot = P.one_gpu_geometry(plan, chunk, 2, slot_bytes, 16, 0, max_ctas)
+    assert -(-slice_elems // tile) < P.K_MAX_ITERATIONS and tile % 8 == 0 and tile * 2 * count <= slot
+
+
+@pytest.mark.parametrize('coll,body', [(AllToAll, alltoall_direct), (AllGather, allgather_direct)])
+@pytest.mark.parametrize('chunk,esize,direct', [(1, 4, True), (333333, 2, True), (1 << 21, 2, True), (1 << 21, 2, False), (1 << 24, 4, True)])
+def test_geometry_of_single_hop_programs(coll, body, chunk, esize, direct):
+    prog = MSCCLProgram('p', fully_connected(8), coll(8, 1, False), 1)
+    with prog:
+        body(8)
+    slot_bytes = 4 << 20
+    plan = P.compile_plan(P.split_copies(load_xml(prog.generate_xml()), 296), range(8), slot_bytes)
+    assert plan.single_hop
+    width = P.access_width(chunk, esize)
+    ctas, streams, slice_elems, tile, slot = P.one_gpu_geometry(plan, chunk, esize, slot_bytes, width, 0, 592, direct)
+    slices = ctas * streams
+    assert ctas * plan.total_tbs() <= 592 and (ctas - 1) * streams * slice_elems < chunk <= slices * slice_elems
+    assert slot * slices <= slot_bytes and 0 < tile <= slice_elems and tile * esize % width == 0 and tile * esize * plan.max_cnt <= slot
+    if direct:
+        assert streams == 1 and tile == min(slice_elems, slot // (plan.max_cnt * width) * (width // esize))
