@@ -596,6 +596,8 @@ def one_gpu_geometry(plan: HostPlan, chunk_elems: int, elem_size: int, slot_byte
     ``tile_elems`` through its own FIFO slots; in one tile when every tile is stored straight into its final slot and no
     step waits for it (all-to-all of 32 MB, copies still behind sends: 153 us in tiles of 128 KB, 141 whole)."""
     per_access = width // elem_size
+    if chunk_elems < 1:
+        raise PlanError('the buffers hold less than one element per chunk')
     if (chunk_elems * elem_size) % width:
         raise PlanError(f'chunks of {chunk_elems * elem_size} bytes are not whole {width}-byte accesses')
     tbs = max(plan.total_tbs(), 1)

@@ -213,3 +213,9 @@ def test_geometry_of_single_hop_programs(coll, body, chunk, esize, direct):
     assert slot * slices <= slot_bytes and 0 < tile <= slice_elems and tile * esize % width == 0 and tile * esize * plan.max_cnt <= slot
     if direct:
         assert streams == 1 and tile == min(slice_elems, slot // (plan.max_cnt * width) * (width // esize))
+
+
+def test_empty_buffers_are_refused():
+    plan = P.compile_plan(_program('two_shot', 4), range(4), 64 << 10)
+    with pytest.raises(P.PlanError):
+        P.one_gpu_geometry(plan, 0, 2, 64 << 10, 2, 0, 592)
