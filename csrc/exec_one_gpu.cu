@@ -586,8 +586,9 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
             if (sk.type == ST_RE && (static_cast<long long>(sk.srcoff) + sk.cnt) * C > me.buf_elems[sk.srcbuf]) { in_bounds = false; worst = sk.srcoff; }
           }
         }
-        if (!in_bounds) {
-          if (gl == 0) record_failure(sync, STATUS_BOUNDS, my_rank, my_tb, s + g, it, st.type, static_cast<unsigned int>(worst));
+        // the lane that records raises the flag: the signal warp, which reports a timeout when it sees it, comes second
+        if (!in_bounds && gl == 0) {
+          record_failure(sync, STATUS_BOUNDS, my_rank, my_tb, s + g, it, st.type, static_cast<unsigned int>(worst));
           *reinterpret_cast<volatile int*>(&sh.fail) = 1;
         }
 

@@ -96,3 +96,34 @@ def test_folded_reduces(name, ranks, protocol):
 def test_small_fifos_and_flag_protocols():
     for protocol in ('LL', 'LL128'):
         _check(_algo('ring', 4, protocol), 40008, torch.float16, fifo_bytes=1 << 20)
+
+
+def test_bounds_failure_is_reported_as_such_by_every_slice(monkeypatch):
+    """Four slices per CTA: the slice that finds its step outside the declared buffer says so before any other warp of the CTA can
+    report that it gave up.  The tensor is larger than declared, so nothing outside owned memory is named."""
+    from msccl.runtime import Communicator, Executor, ExecutorError
+    import msccl.runtime.plan as P
+    monkeypatch.setattr(P, 'ONE_GPU_TILE_BYTES', 2048)
+    chunk, algo = 65536, _algo('ring', 4, 'Simple')
+    comm = Communicator.emulated(4, fifo_bytes=8 << 20)
+    try:
+        ex = Executor(comm)
+        plan = ex.compile(algo)
+        for _ in range(3):
+            comm.timeout_ns = int(0.5e9)                       # the other ranks wait this long for the rank that stopped
+            ins = {r: torch.full((4 * chunk,), float(r + 1), device='cuda') for r in range(4)}
+            ex.run(plan, ins, declared_elems={r: ((3 if r == 2 else 4) * chunk, 0, 0) for r in range(4)})
+            with pytest.raises(ExecutorError):
+                ex.check()
+            status = comm.native.read_status(comm.sync_ptr(2))
+            assert status[0] == 6 and status[1] == 2           # STATUS_BOUNDS, reported by rank 2
+            comm.reset_after_failure()
+            comm.timeout_ns = int(20e9)
+            ins = {r: torch.full((4 * chunk,), float(r + 1), device='cuda') for r in range(4)}
+            out = ex.run(plan, ins)
+            ex.check()
+            assert all(torch.all(out[r] == 10) for r in range(4))
+        assert next(iter(plan.geometry.values()))[1] == 4
+        plan.close()
+    finally:
+        comm.close()
