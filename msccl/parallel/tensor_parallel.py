@@ -37,9 +37,14 @@ class TensorParallelMLP:
         self.w_gate_up = interleave_gate_up(w_gate, w_up)
         self.w_down = mk(hidden, self.shard) if w_down is None else w_down.contiguous()
         self.fused = FusedTensorParallel(comm, tokens_per_rank, hidden)
-        self.h = torch.empty(comm.world * tokens_per_rank, self.shard, dtype=torch.bfloat16, device=dev)
-        # MSCCL_FUSED_PAIR=0 asks for the fused single-CTA kernels whatever the number of ranks
-        self.plain = comm.world == 1 and os.environ.get('MSCCL_FUSED_PAIR', '1') != '0'
+        # MSCCL_FUSED_PAIR=0 asks for the fused single-CTA kernels whatever the number of ranks; MSCCL_GEMM_PAIR=0 takes the plain
+        # GEMMs off the CTA pairs that make them the faster choice (the quantising epilogue exists on pairs only)
+        self.plain = (comm.world == 1 and os.environ.get('MSCCL_FUSED_PAIR', '1') != '0'
+                      and os.environ.get('MSCCL_GEMM_PAIR', '1') == '1')
+        # SwiGLU of the last call; with the quantising epilogue it exists as h_q and h_sf only
+        self.h = None
+        if not (self.plain and precision == 'mxfp8'):
+            self.h = torch.empty(comm.world * tokens_per_rank, self.shard, dtype=torch.bfloat16, device=dev)
         if precision == 'mxfp8':
             if self.plain:
                 self.h_q = torch.empty(tokens_per_rank, self.shard, dtype=torch.float8_e4m3fn, device=dev)
@@ -59,7 +64,7 @@ class TensorParallelMLP:
                 out = torch.empty(rows, hidden, dtype=torch.bfloat16, device=x_local.device)
             assert out.is_contiguous()
             y = out.view(-1).view(torch.bfloat16)[:rows * hidden].view(rows, hidden)      # any contiguous memory of that size will do
-            self.fused.launches += 2
+            self.fused.launches += 3 if self.precision == 'mxfp8' else 2
             if self.precision == 'mxfp8':
                 xq, sx = quantize_mxfp8_packed(x_local)
                 hq, sh = gemm_mxfp8_swiglu(xq, sx, self.wq_gate_up, self.sf_gate_up, self.h_q, self.h_sf)
