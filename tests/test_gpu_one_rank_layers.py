@@ -1,4 +1,5 @@
-"""The layers on one GPU (a communicator of one process): the MLP that runs on the plain GEMM kernels there."""
+"""The layers on one GPU (a communicator of one process): the MLP that runs on the plain GEMM kernels there, and the GEMM
+epilogue that quantises its SwiGLU result."""
 import os
 
 import pytest
@@ -98,3 +99,54 @@ def test_switches_take_the_layer_back_to_the_fused_kernels(one_rank, switch, pre
         assert torch.equal(got, plain)
     else:                                              # the plain kernels split K here: bits may differ by a rounding
         assert float((got.double() - plain.double()).norm() / plain.double().norm()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize('tokens', [128, 256, 384, 1024])
+def test_quantised_swiglu_gives_the_bytes_of_the_separate_kernels(one_rank, tokens):
+    """The fused all-gather GEMM on one rank stores the bf16 SwiGLU, which the quantisation kernel then reads."""
+    from msccl.ops import check_gemm_errors
+    from msccl.ops.fused_tp import FusedTensorParallel
+    from msccl.ops.gemm import gemm_mxfp8_swiglu, interleave_gate_up, pack_mx_scales, quantize_mxfp8, quantize_mxfp8_packed
+    hidden, ffn = 1024, 1280
+    gen = torch.Generator(device='cuda').manual_seed(tokens)
+    w_gate, w_up, _ = _weights(gen, hidden, ffn)
+    x = _normal(gen, tokens, hidden) * torch.exp2(torch.randint(-8, 9, (tokens, 1), device='cuda', generator=gen).float()).bfloat16()
+    fused = FusedTensorParallel(one_rank(tokens * hidden * 8 + (4 << 20)), tokens, hidden)
+    packed = {}
+    for tile in (256, fused.mx_gate_up_tile):
+        q, s = quantize_mxfp8(interleave_gate_up(w_gate, w_up, tile=tile).float())
+        packed[tile] = q, pack_mx_scales(s, row_multiple=128)
+    xq, sx = quantize_mxfp8_packed(x)
+    want_q, want_sf = quantize_mxfp8_packed(fused.all_gather_gemm_mxfp8(xq, sx, *packed[fused.mx_gate_up_tile], epilogue='swiglu'))
+    q = torch.empty(tokens, ffn, dtype=torch.float8_e4m3fn, device='cuda')
+    sf = torch.empty(tokens // 128 * (ffn // 128) * 512, dtype=torch.uint8, device='cuda')
+    gemm_mxfp8_swiglu(xq, sx, *packed[256], q, sf)
+    check_gemm_errors()
+    assert torch.equal(q.view(torch.uint8), want_q.view(torch.uint8)) and torch.equal(sf, want_sf)
+
+
+@pytest.mark.parametrize('m', [1, 130, 257])
+def test_quantised_swiglu_writes_its_rows_only(m):
+    from msccl.ops import check_gemm_errors
+    from msccl.ops.gemm import gemm_mxfp8_swiglu, quantize_mxfp8_packed
+    n, k, padded = 1024, 512, -(-m // 256) * 256
+    gen = torch.Generator(device='cuda').manual_seed(m)
+    a, b = _normal(gen, padded, k), _normal(gen, n, k, std=0.05)
+    bq, sb = quantize_mxfp8_packed(b)
+    full_q = torch.empty(padded, n // 2, dtype=torch.float8_e4m3fn, device='cuda')
+    full_sf = torch.empty(padded // 128 * (n // 256) * 512, dtype=torch.uint8, device='cuda')
+    gemm_mxfp8_swiglu(*quantize_mxfp8_packed(a), bq, sb, full_q, full_sf)
+    q = torch.full((m + 2, n // 2), 85, dtype=torch.uint8, device='cuda')
+    blocks = -(-m // 128) * (n // 256)
+    sf = torch.full(((blocks + 2) * 512,), 255, dtype=torch.uint8, device='cuda')
+    gemm_mxfp8_swiglu(*quantize_mxfp8_packed(a[:m]), bq, sb, q[1:-1].view(torch.float8_e4m3fn), sf[512:-512])
+    check_gemm_errors()
+    assert torch.equal(q[1:-1], full_q[:m].view(torch.uint8)) and torch.all(q[0] == 85) and torch.all(q[-1] == 85)
+    assert torch.all(sf[:512] == 255) and torch.all(sf[-512:] == 255)
+    # byte (r % 32) * 16 + (r // 32) * 4 + j of a block is row r's
+    byte = torch.arange(512, device='cuda')
+    row = byte // 16 + byte % 16 // 4 * 32
+    got, want = sf[512:-512].view(-1, n // 256, 512), full_sf.view(-1, n // 256, 512)
+    for block in range(got.shape[0]):
+        mine = row + 128 * block < m
+        assert torch.equal(got[block][:, mine], want[block][:, mine]) and torch.all(got[block][:, ~mine] == 255)
