@@ -25,6 +25,7 @@ struct alignas(128) FusedPage {
   unsigned long long moe_base[kFusedMaxRanks];                     // local: moe_count at the end of the previous launch
   unsigned long long moe_epoch;
   unsigned int moe_done, moe_pad;
+  unsigned int moe_claimed, moe_moved;                             // local, one rank: token copies taken / stored by a running dispatch
 };
 
 struct AgGemmArgs {

@@ -44,7 +44,7 @@ moe_dispatch_gemm_kernel(const __grid_constant__ CUtensorMap map_a0, const __gri
 
   if (static_cast<int>(blockIdx.x) < g.comm_ctas) {
     // ---------------------------------------------------------------- comm CTAs
-    moe_comm_role(g, page, epoch, parity, &sh, p.abort_flag, g.comm_ctas);
+    moe_comm_role(g, page, epoch, parity, &sh, p.abort_flag);
   } else {
     // ---------------------------------------------------------------- GEMM CTAs
     init_pipe(p);

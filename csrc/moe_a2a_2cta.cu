@@ -37,9 +37,8 @@ moe_dispatch_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a0, const 
   const uint32_t cta_rank = cluster_ctarank();
   const bool leader = cta_rank == 0;
   const int cluster = static_cast<int>(cluster_id_x()), clusters = static_cast<int>(num_clusters_x());
-  // One rank: the dispatch is a gather inside this GPU's memory, with no transfer to overlap.  Every CTA takes its share
-  // of it and then runs tiles, instead of 16 CTAs moving all rows while the others wait and then standing by (4096
-  // tokens, 8 experts, top-2: 1650 us with 66 pairs for the tiles).
+  // One rank: every CTA moves rows (moe_gather_role) and then runs tiles, instead of 16 CTAs moving all of them while the
+  // others wait and then standing by (4096 tokens, 8 experts, top-2: 1650 us with 66 pairs for the tiles, 1432 this way).
   const bool everyone = g.nranks == 1;
   const int comm_clusters = everyone ? 0 : g.comm_ctas / 2;
   bool skip = false;
@@ -49,7 +48,7 @@ moe_dispatch_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a0, const 
     skip = g.error_words != nullptr && *reinterpret_cast<volatile int*>(g.error_words) != 0;
     if (threadIdx.x == 0) *p.abort_flag = 0;
     __syncthreads();
-    if (!skip) moe_comm_role(g, page, epoch, parity, &sh, p.abort_flag, g.comm_ctas);
+    if (!skip) moe_comm_role(g, page, epoch, parity, &sh, p.abort_flag);
   } else {
     // ---------------------------------------------------------------- GEMM pairs
     if (threadIdx.x == 0) s_skip = (g.error_words != nullptr && *reinterpret_cast<volatile int*>(g.error_words) != 0) ? 1 : 0;
@@ -61,7 +60,7 @@ moe_dispatch_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a0, const 
     tc_fence_after_sync();
     const uint32_t tmem_base = *p.tmem_slot;
     skip = ld_shared_cluster_u32(map_to_cta(smem_u32(&s_skip), 0)) != 0;      // the leader's reading decides for the pair
-    if (everyone && !skip) moe_comm_role(g, page, epoch, parity, &sh, p.abort_flag, static_cast<int>(gridDim.x));
+    if (everyone && !skip) moe_gather_role(g, page, epoch, parity, &sh, p.abort_flag);
     const bool have_counts = !skip && load_counts(g, page, epoch, parity, &sh, p.abort_flag);
     const int pairs = clusters - comm_clusters, pair = cluster - comm_clusters;
     const int n_out = 2 * g.ffn, tiles_n = n_out / PBN, k_blocks = g.hidden / BK;
@@ -169,6 +168,8 @@ moe_dispatch_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a0, const 
     __threadfence();
     if (atomicAdd(&page->moe_done, 1u) == gridDim.x - 1u) {
       page->moe_done = 0;
+      page->moe_claimed = 0;
+      page->moe_moved = 0;
       page->moe_pad = 1;                                         // the epoch advances after the second kernel
     }
   }

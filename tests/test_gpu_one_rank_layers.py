@@ -1,5 +1,5 @@
-"""The layers on one GPU (a communicator of one process): the MLP that runs on the plain GEMM kernels there, and the GEMM
-epilogue that quantises its SwiGLU result."""
+"""The layers on one GPU (a communicator of one process): the MLP that runs on the plain GEMM kernels there, the GEMM epilogue
+that quantises its SwiGLU result, and the MoE dispatch in which every CTA moves rows."""
 import os
 
 import pytest
@@ -150,3 +150,57 @@ def test_quantised_swiglu_writes_its_rows_only(m):
     for block in range(got.shape[0]):
         mine = row + 128 * block < m
         assert torch.equal(got[block][:, mine], want[block][:, mine]) and torch.all(got[block][:, ~mine] == 255)
+
+
+def _moe_reference(x, logits, topk, layer, hidden, ffn):
+    from msccl.ops.moe import route_top_k
+    experts, weights = route_top_k(logits, topk)
+    want = torch.zeros(x.shape[0], hidden, dtype=torch.float64, device='cuda')
+    gate_up = layer.w_gate_up.view(-1, ffn // 128, 2, 128, hidden).double()
+    down = layer.w_down.view(-1, hidden, ffn).double()
+    for e in range(down.shape[0]):
+        gate, up = (gate_up[e, :, i].reshape(ffn, hidden) for i in (0, 1))
+        h = _swiglu(x.double() @ gate.t(), x.double() @ up.t()).bfloat16().double()
+        share = torch.where(experts == e, weights.double(), 0).sum(1, keepdim=True)
+        want += share * (h @ down[e].t())
+    return want
+
+
+@pytest.mark.parametrize('tokens,topk', [(1, 1), (5, 2), (6, 1), (130, 2), (1776, 2), (1777, 2), (4100, 1)])
+def test_moe_dispatch_by_every_cta(one_rank, tokens, topk):
+    """Fewer copies than one batch, a short last batch, both sides of the line between one and two copies per warp (4 x 6 x 148
+    copies), several calls: the counters start again.  The products of an expert are rounded to bf16 before the sum over the
+    experts and the sum once more, 2^-8 together, and the intermediate rounding adds less than 2^-10 (see the MLP test)."""
+    from msccl.ops import check_gemm_errors
+    from msccl.parallel import ExpertParallelMoE
+    hidden, ffn, experts = 256, 256, 8
+    comm = one_rank((2 * tokens * topk + 2048 + tokens * topk) * hidden * 4 + (4 << 20))
+    layer = ExpertParallelMoE(comm, tokens, hidden, ffn, experts, topk, seed=3)
+    gen = torch.Generator(device='cuda').manual_seed(tokens)
+    for _ in range(4):
+        x, logits = _normal(gen, tokens, hidden), torch.randn(tokens, experts, device='cuda', generator=gen)
+        got = layer(x, gate_logits=logits)
+        check_gemm_errors()
+        want = _moe_reference(x, logits, topk, layer, hidden, ffn)
+        assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8 + 2.0 ** -10
+        assert torch.equal(layer(x, gate_logits=logits), got)
+
+
+def test_moe_beside_another_stream(one_rank):
+    """CTAs that another stream's kernels keep off the GPU have no share of the rows that the others wait for."""
+    from msccl.ops import check_gemm_errors
+    from msccl.parallel import ExpertParallelMoE
+    tokens, hidden, ffn = 1024, 512, 512
+    layer = ExpertParallelMoE(one_rank((3 * tokens * 2 + 2048) * hidden * 4 + (4 << 20)), tokens, hidden, ffn, 8, 2, seed=4)
+    gen = torch.Generator(device='cuda').manual_seed(9)
+    x, logits = _normal(gen, tokens, hidden), torch.randn(tokens, 8, device='cuda', generator=gen)
+    want = layer(x, gate_logits=logits)
+    a = _normal(gen, 4096, 4096)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        products = [a @ a for _ in range(40)]
+    got = [layer(x, gate_logits=logits) for _ in range(10)]
+    torch.cuda.synchronize()
+    check_gemm_errors()
+    assert all(torch.equal(t, want) for t in got) and all(torch.equal(t, products[0]) for t in products)
