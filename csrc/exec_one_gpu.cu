@@ -38,6 +38,10 @@ constexpr int kOgSmemSteps = 128;
 
 enum JobKind : int { JOB_EXIT = 0, JOB_NONE, JOB_MOVE, JOB_BATCH, JOB_SEND, JOB_RECV, JOB_BOTH };
 
+// A flag-in-data poll that ran out of time leaves its report to the signal warp; whoever in the control warp raises the flag
+// reports by itself (and the signal warp, which may see the flag first, must not call that a timeout).
+enum FailKind : int { FAIL_REPORTED = 1, FAIL_DATA = 2 };
+
 struct __align__(16) Job {
   const char* in;                 // local source / destination slot already holding the data / FIFO packets
   const char* add;                // second operand or null
@@ -59,7 +63,7 @@ struct __align__(16) Job {
 struct Shared {
   Job job[2];
   unsigned long long go[2], done[2];     // mbarriers
-  int fail;                              // a flag-in-data poll or a wait ran out of time
+  int fail;                              // FAIL_*: everybody gives up
   int leave;                             // the first data warp waited too long for a job: all leave
   int signalled;                         // passes the signal warp has finished with
   DevStep steps[kOgSmemSteps];
@@ -247,7 +251,7 @@ __device__ __forceinline__ void og_move_ll(const char* in, const char* add1, cha
         for (int u = 0; u < U; ++u) ready = ready && pk[u].ready(flag_in);
         if (ready) break;
         if ((spins & 127u) == 0 && (*reinterpret_cast<volatile int*>(fail) != 0 || w.expired())) {
-          *reinterpret_cast<volatile int*>(fail) = 1;
+          *reinterpret_cast<volatile int*>(fail) = FAIL_DATA;
           break;
         }
       }
@@ -299,7 +303,7 @@ __device__ __forceinline__ void og_move_ll128(const char* in, const char* add1, 
         if ((spins & 63u) == 0) {
           const bool give_up = (threadIdx.x & 31) == 0 && (*reinterpret_cast<volatile int*>(fail) != 0 || w.expired());
           if (__any_sync(kFullWarp, give_up)) {
-            *reinterpret_cast<volatile int*>(fail) = 1;
+            *reinterpret_cast<volatile int*>(fail) = FAIL_DATA;
             break;
           }
         }
@@ -409,8 +413,10 @@ __device__ __forceinline__ void signal_role(Shared& sh, SyncPage* sync, int rank
     if (job.kind == JOB_EXIT) return;
     unsigned long long moved = 0;
     if (trace != nullptr) moved = global_timer_ns();
-    if (*reinterpret_cast<volatile int*>(&sh.fail) != 0) {
-      record_failure(sync, STATUS_TIMEOUT_DATA, rank, tb, job.step, job.iter, recv_peer, chan);   // the first failure recorded wins
+    const int fail = *reinterpret_cast<volatile int*>(&sh.fail);
+    if (fail != 0) {
+      // the first failure recorded wins
+      if (fail == FAIL_DATA) record_failure(sync, STATUS_TIMEOUT_DATA, rank, tb, job.step, job.iter, recv_peer, chan);
     } else {
       // one fence covers everything the step publishes; the credit alone needs none (the data warps have used what they
       // read from the FIFO slot before they came to the barrier)
@@ -586,10 +592,9 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
             if (sk.type == ST_RE && (static_cast<long long>(sk.srcoff) + sk.cnt) * C > me.buf_elems[sk.srcbuf]) { in_bounds = false; worst = sk.srcoff; }
           }
         }
-        // the lane that records raises the flag: the signal warp, which reports a timeout when it sees it, comes second
-        if (!in_bounds && gl == 0) {
-          record_failure(sync, STATUS_BOUNDS, my_rank, my_tb, s + g, it, st.type, static_cast<unsigned int>(worst));
-          *reinterpret_cast<volatile int*>(&sh.fail) = 1;
+        if (!in_bounds) {
+          if (gl == 0) record_failure(sync, STATUS_BOUNDS, my_rank, my_tb, s + g, it, st.type, static_cast<unsigned int>(worst));
+          *reinterpret_cast<volatile int*>(&sh.fail) = FAIL_REPORTED;
         }
 
         // lane 0 of the group: a free FIFO slot; 1: the tile; 2: may the tile go straight into the receiver's slot? (looked
@@ -648,7 +653,7 @@ __global__ void __launch_bounds__(kOgThreads, kOgCtasPerSm) exec_one_gpu_kernel(
               else if (gl >= 3) { const DevStep& sk = sp[s + dep - (LP - 3)]; code = STATUS_TIMEOUT_DEP; aux0 = sk.depid; aux1 = sk.deps; }
             }
             record_failure(sync, code, my_rank, my_tb, s + g, it, aux0, aux1);
-            *reinterpret_cast<volatile int*>(&sh.fail) = 1;
+            *reinterpret_cast<volatile int*>(&sh.fail) = FAIL_REPORTED;
           }
           __syncwarp();
           break;

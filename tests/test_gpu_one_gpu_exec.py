@@ -127,3 +127,35 @@ def test_bounds_failure_is_reported_as_such_by_every_slice(monkeypatch):
         plan.close()
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize('protocol', ['Simple', 'LL', 'LL128'])
+def test_a_receive_that_nothing_feeds_is_reported_as_such(protocol, monkeypatch):
+    """Under Simple the control warp waits for the tile, under LL and LL128 the data warps poll its packets: either way the
+    (short) wait ends in the same status, and the device stays usable."""
+    from msccl.runtime import Communicator, Executor, ExecutorError
+    import msccl.runtime.executor as executor
+    lonely = load_xml(f'<algo name="lonely" proto="{protocol}" nchannels="1" nchunksperloop="1" ngpus="2" coll="custom" inplace="0">'
+                      '<gpu id="0" i_chunks="1" o_chunks="1" s_chunks="0"><tb id="0" send="-1" recv="1" chan="0">'
+                      '<step s="0" type="r" srcbuf="i" srcoff="0" dstbuf="o" dstoff="0" cnt="1" depid="-1" deps="-1" hasdep="0"/>'
+                      '</tb></gpu><gpu id="1" i_chunks="1" o_chunks="1" s_chunks="0"></gpu></algo>')
+    comm = Communicator.emulated(2, fifo_bytes=1 << 20)
+    try:
+        comm.timeout_ns = int(0.2e9)
+        ex = Executor(comm)
+        checked = executor.compile_plan
+        with monkeypatch.context() as patch:
+            patch.setattr(executor, 'compile_plan', lambda algo, ranks, slot: checked(algo, ranks, slot, check=False))
+            plan = ex.compile(lonely)
+        ex.run(plan, {r: torch.ones(1024, device='cuda') for r in range(2)})
+        with pytest.raises(ExecutorError) as err:
+            ex.check()
+        assert err.value.code == 2 and err.value.rank == 0 and err.value.aux0 == 1      # STATUS_TIMEOUT_DATA, waiting for rank 1
+        comm.reset_after_failure()
+        comm.timeout_ns = int(20e9)
+        ins = {r: torch.full((2 * 1024,), float(r + 1), device='cuda') for r in range(2)}
+        ex.run(ex.compile(_algo('ring', 2, protocol)), ins)
+        ex.check()
+        assert all(torch.all(ins[r] == 3) for r in range(2))
+    finally:
+        comm.close()
