@@ -25,7 +25,7 @@ import torch
 
 from msccl.runtime.comm import Communicator
 from msccl.runtime.plan import (HostPlan, PlanError, access_width, chunk_geometry, compile_plan, fold_reduce_chains,
-                                one_gpu_geometry, split_copies, tile_geometry, K_FIFO_SLOTS)
+                                occupy_idle_ranks, one_gpu_geometry, split_copies, tile_geometry, K_FIFO_SLOTS)
 from msccl.xml.loader import AlgoIR, load_plan_table, load_xml
 
 DTYPE_CODES = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
@@ -59,7 +59,7 @@ class DevicePlan:
             raise PlanError('FIFO area too small for this program')
         # with every rank on this GPU a hop between threadblocks costs more than the add it passes on
         if comm.emulated_mode:
-            algo = split_copies(fold_reduce_chains(algo), most_tbs=2 * comm.native.sm_count())
+            algo = split_copies(fold_reduce_chains(occupy_idle_ranks(algo)), most_tbs=2 * comm.native.sm_count())
         self.host: HostPlan = compile_plan(algo, comm.local_ranks, self.slot_bytes)
         self.geometry = {}         # emulated mode: (chunk elements, dtype, width, direct) -> launch geometry
         self.rank_info = [(self.host.extents[r]['i'], self.host.extents[r]['o'], self.host.extents[r]['s'], algo.gpus[r].o_chunks,

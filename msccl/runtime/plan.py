@@ -24,7 +24,7 @@ from dataclasses import dataclass, field, replace
 from itertools import count
 from typing import Dict, List
 
-from msccl.xml.loader import AlgoIR, StepIR
+from msccl.xml.loader import AlgoIR, StepIR, TbIR
 from msccl.xml.validator import validate
 
 STEP_CODES = {'nop': 0, 's': 1, 'r': 2, 'rcs': 3, 'rrs': 4, 'rrc': 5, 'rrcs': 6, 'cpy': 7, 're': 8}
@@ -220,6 +220,18 @@ def _batches(tb):
     return out
 
 
+_NOP = StepIR(0, 'nop', 'i', -1, 'o', -1, 0, -1, -1, False)
+
+
+def occupy_idle_ranks(algo: AlgoIR) -> AlgoIR:
+    """The program with a threadblock that does nothing on every rank that has none.  The last threadblock of a rank advances the
+    rank's launch epoch, which the packet flags of LL and LL128 are made of: a rank that sat a launch out would never find the
+    flags of its peers again."""
+    if all(g.tbs for g in algo.gpus):
+        return algo
+    return replace(algo, gpus=[g if g.tbs else replace(g, tbs=[TbIR(0, -1, -1, 0, [replace(_NOP)])]) for g in algo.gpus])
+
+
 def _dependencies_exist(gpu):
     """False: the validator will report the program, which is left as it is."""
     return all(st.depid < 0 or (st.depid < len(gpu.tbs) and 0 <= st.deps < len(gpu.tbs[st.depid].steps))
@@ -276,9 +288,6 @@ def split_copies(algo: AlgoIR, most_tbs: int) -> AlgoIR:
 
 def _overlap(o1, c1, o2, c2):
     return o1 < o2 + c2 and o2 < o1 + c1
-
-
-_NOP = StepIR(0, 'nop', 'i', -1, 'o', -1, 0, -1, -1, False)
 
 
 class _Node:

@@ -159,3 +159,29 @@ def test_a_receive_that_nothing_feeds_is_reported_as_such(protocol, monkeypatch)
         assert all(torch.all(ins[r] == 3) for r in range(2))
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize('protocol', ['LL', 'LL128', 'Simple'])
+def test_a_rank_without_threadblocks_keeps_up_with_the_others(protocol):
+    """Flags of LL and LL128 packets name the launch: a rank with nothing to do in one launch counts it all the same."""
+    from msccl.runtime import Communicator, Executor
+    step = '<step s="0" type="{}" srcbuf="i" srcoff="0" dstbuf="i" dstoff="0" cnt="1" depid="-1" deps="-1" hasdep="0"/>'
+    gpu = '<gpu id="{}" i_chunks="1" o_chunks="0" s_chunks="0">{}</gpu>'
+    head = '<algo name="pair" proto="LL" nchannels="1" nchunksperloop="1" ngpus="3" coll="custom" inplace="1">'
+    pair = load_xml(head + gpu.format(0, '<tb id="0" send="1" recv="-1" chan="0">' + step.format('s') + '</tb>') +
+                    gpu.format(1, '<tb id="0" send="-1" recv="0" chan="0">' + step.format('rrc') + '</tb>') + gpu.format(2, '') + '</algo>')
+    comm = Communicator.emulated(3, fifo_bytes=1 << 20)
+    try:
+        comm.timeout_ns = int(2e9)
+        ex = Executor(comm)
+        plans = ex.compile(pair), ex.compile(_algo('ring', 3, protocol))
+        for _ in range(3):
+            ins = {r: torch.full((3 * 1024,), float(r + 1), device='cuda') for r in range(3)}
+            ex.run(plans[0], ins)
+            ex.check()
+            assert [float(ins[r][5]) for r in range(3)] == [1, 3, 3]
+            ex.run(plans[1], ins)
+            ex.check()
+            assert all(torch.all(ins[r] == 7) for r in range(3))
+    finally:
+        comm.close()

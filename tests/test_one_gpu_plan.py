@@ -219,3 +219,12 @@ def test_empty_buffers_are_refused():
     plan = P.compile_plan(_program('two_shot', 4), range(4), 64 << 10)
     with pytest.raises(P.PlanError):
         P.one_gpu_geometry(plan, 0, 2, 64 << 10, 2, 0, 592)
+
+
+def test_every_rank_has_a_threadblock():
+    algo = _wide(1)
+    idle = replace(algo, ngpus=3, gpus=algo.gpus + [replace(algo.gpus[0], id=2, tbs=[])])
+    assert P.occupy_idle_ranks(algo) is algo
+    filled = P.occupy_idle_ranks(idle)
+    assert validate(filled) == [] and not idle.gpus[2].tbs and [len(g.tbs) for g in filled.gpus] == [1, 1, 1]
+    assert P.compile_plan(filled, range(3), 64 << 10).num_tbs == {0: 1, 1: 1, 2: 1}
