@@ -188,7 +188,9 @@ def _open_positions(algo: AlgoIR, match):
 
 def _batches(tb):
     """``{first step index: number of steps}`` for runs of ``re`` steps into one destination (``nop`` steps may sit
-    between them) that the kernel executes as one multi-input add."""
+    between them) that the kernel executes as one multi-input add: it waits for everything the steps wait for, then adds.
+    So behind a step that somebody waits for no step of the run may wait: what it waits for could be ordered after that step
+    (the source refilled, say, once the first add has read it), and the add would wait for itself."""
     out = {}
     steps = tb.steps
     i = 0
@@ -197,10 +199,13 @@ def _batches(tb):
         if st.type != 're':
             i += 1
             continue
-        j, last_re, sources = i + 1, i, 1
+        j, last_re, sources, awaited = i + 1, i, 1, False
         srcs = {(st.srcbuf, st.srcoff)}
         while j < len(steps) and sources < K_MAX_BATCH and j - i < 2 * K_MAX_BATCH:
             nx = steps[j]
+            awaited = awaited or steps[j - 1].hasdep
+            if awaited and nx.depid >= 0:
+                break
             if nx.type == 'nop':
                 j += 1
                 continue

@@ -16,6 +16,7 @@ from msccl.programs.allgather import allgather_direct
 from msccl.programs.allreduce import allreduce_allpairs, allreduce_ring
 from msccl.xml import load_xml
 from test_gpu_executor import _cases, _program
+from test_plan_compile import refilled_source
 
 pytestmark = pytest.mark.gpu
 DTYPES = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
@@ -264,3 +265,22 @@ def test_both_interpreters_share_a_communicator(emulated):
     for plan, run in plans:
         plan.close()
         run.close()
+
+
+@pytest.mark.parametrize('protocol', ['Simple', 'LL', 'LL128'])
+def test_adds_whose_source_is_refilled_between_them(emulated, protocol):
+    """Two adds into one slot, the second of which waits for what comes after the first: not one multi-input add, in either kernel."""
+    from msccl.runtime import Executor
+    algo = _program('refilled', AllReduce(2, 1, True), lambda: refilled_source(5), threadblock_policy=ThreadblockPolicy.manual,
+                    protocol=protocol)
+    comm = emulated(2, 1 << 20)
+    comm.timeout_ns = int(2e9)
+    ex, run = Executor(comm), Launcher(comm, algo)
+    plan = ex.compile(algo)
+    for launch in (lambda ins: ex.run(plan, ins), run):
+        ins = {r: torch.full((5000,), float(r + 1), device='cuda') for r in range(2)}
+        launch(ins)
+        ex.check()
+        assert torch.all(ins[0] == 1) and torch.all(ins[1] == 7)
+    plan.close()
+    run.close()

@@ -3,13 +3,16 @@ tile geometry and limits) and the table checks of the allocation-free entry poin
 the entry point rejects bad tables before it makes its first CUDA call."""
 import ctypes
 import struct
+from dataclasses import replace
 
 import pytest
+import torch
 
-from msccl.language import MSCCLProgram, ThreadblockPolicy
+from msccl.interp import input_chunks_of, run_algorithm
+from msccl.language import Buffer, MSCCLProgram, ThreadblockPolicy, chunk
 from msccl.language.collectives import AllGather, AllReduce, AllToAll
 from msccl.programs.allgather import allgather_direct, allgather_ring
-from msccl.programs.allreduce import allreduce_allpairs, allreduce_ring, allreduce_two_shot
+from msccl.programs.allreduce import allreduce_allpairs, allreduce_one_shot, allreduce_ring, allreduce_two_shot
 from msccl.programs.alltoall import alltoall_direct
 from msccl.runtime import plan as P
 from msccl.topologies import fully_connected
@@ -189,3 +192,60 @@ def test_noalloc_entry_point_rejects_inconsistent_tables():
     assert _call(lib, tbs, steps, n, scratch, proto=5) == BAD
     assert _call(lib, tbs, steps, n, scratch, slot=1000) == BAD
     assert _call(lib, tbs, steps, n, scratch, chunk=3, proto=2) == BAD
+
+
+def refilled_source(rounds=2):
+    """Rank 1 adds what it receives into one scratch slot, ``rounds`` times, in another threadblock than the one that receives: a
+    receive waits for the add before, the next add for the receive."""
+    for _ in range(rounds):
+        chunk(0, Buffer.input, 0).copy(1, 's', 0, sendtb=0, recvtb=0, ch=0)
+        chunk(1, Buffer.input, 0).reduce(chunk(1, 's', 0), sendtb=1, ch=0)
+
+
+def _batches_as_one_step(algo):
+    """What the kernels make of a program: a batch waits for everything its steps wait for, and whoever waits for one of its steps
+    waits for the last."""
+    gpus = []
+    for g in algo.gpus:
+        fresh, at = [], {}
+        for t, tb in enumerate(g.tbs):
+            steps, i = [], 0
+            batches = P._batches(tb)
+            while i < len(tb.steps):
+                members = tb.steps[i:i + batches.get(i, 1)]
+                if len(members) > 1:
+                    steps += [replace(st, type='nop', cnt=0, hasdep=False) for st in members if st.depid >= 0]
+                    adds = [replace(st, depid=-1, deps=-1, hasdep=False) for st in members if st.type == 're']
+                    adds[-1].hasdep = any(st.hasdep for st in members)
+                    steps += adds
+                else:
+                    steps.append(replace(members[0]))
+                at.update({(t, i + k): len(steps) - 1 for k in range(len(members))})
+                i += len(members)
+            fresh.append(replace(tb, steps=steps))
+        for tb in fresh:
+            for k, st in enumerate(tb.steps):
+                st.s, st.deps = k, at[st.depid, st.deps] if st.depid >= 0 else -1
+        gpus.append(replace(g, tbs=fresh))
+    return replace(algo, gpus=gpus)
+
+
+@pytest.mark.parametrize('name', ['refilled2', 'refilled5', 'allpairs4', 'allpairs4_nop', 'two_shot4', 'one_shot9', 'one_shot9_folded'])
+def test_batches_never_wait_for_themselves(name):
+    programs = {
+        'refilled2': lambda: _program('r', AllReduce(2, 1, True), refilled_source, threadblock_policy=MANUAL),
+        'refilled5': lambda: _program('r', AllReduce(2, 1, True), lambda: refilled_source(5), threadblock_policy=MANUAL),
+        'allpairs4': lambda: _program('a', AllReduce(4, 16, True), lambda: allreduce_allpairs(4), threadblock_policy=MANUAL),
+        'allpairs4_nop': lambda: _program('a', AllReduce(4, 16, True), lambda: allreduce_allpairs(4), threadblock_policy=MANUAL,
+                                          dependence_nop=True),
+        'two_shot4': lambda: _program('t', AllReduce(4, 4, True), lambda: allreduce_two_shot(4), threadblock_policy=MANUAL),
+        'one_shot9': lambda: _program('o', AllReduce(9, 1, True), lambda: allreduce_one_shot(9), threadblock_policy=MANUAL),
+        'one_shot9_folded': lambda: P.fold_reduce_chains(programs['one_shot9']()),
+    }
+    algo = programs[name]()
+    gen = torch.Generator().manual_seed(2)
+    host = [torch.randn(input_chunks_of(algo, r) * 24, generator=gen).bfloat16() for r in range(algo.ngpus)]
+    want = run_algorithm(algo, host, 24, dtype=torch.bfloat16)
+    got = run_algorithm(_batches_as_one_step(algo), host, 24, dtype=torch.bfloat16, fifo_depth=P.K_FIFO_SLOTS)
+    assert all(torch.equal(a.view(torch.int16), b.view(torch.int16)) for a, b in zip(want, got))
+    assert (sum(len(P._batches(tb)) for g in algo.gpus for tb in g.tbs) > 0) == (name in ('allpairs4', 'allpairs4_nop', 'one_shot9_folded'))
