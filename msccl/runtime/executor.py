@@ -57,9 +57,10 @@ class DevicePlan:
         self.slot_bytes = slot // 1024 * 1024
         if self.slot_bytes < 1024:
             raise PlanError('FIFO area too small for this program')
+        algo = occupy_idle_ranks(algo)
         # with every rank on this GPU a hop between threadblocks costs more than the add it passes on
         if comm.emulated_mode:
-            algo = split_copies(fold_reduce_chains(occupy_idle_ranks(algo)), most_tbs=2 * comm.native.sm_count())
+            algo = split_copies(fold_reduce_chains(algo), most_tbs=2 * comm.native.sm_count())
         self.host: HostPlan = compile_plan(algo, comm.local_ranks, self.slot_bytes)
         self.geometry = {}         # emulated mode: (chunk elements, dtype, width, direct) -> launch geometry
         self.rank_info = [(self.host.extents[r]['i'], self.host.extents[r]['o'], self.host.extents[r]['s'], algo.gpus[r].o_chunks,

@@ -10,7 +10,7 @@ import pytest
 import torch
 
 from msccl.interp import input_chunks_of, run_algorithm
-from msccl.language import ThreadblockPolicy
+from msccl.language import Buffer, ThreadblockPolicy, chunk
 from msccl.language.collectives import AllGather, AllReduce
 from msccl.programs.allgather import allgather_direct
 from msccl.programs.allreduce import allreduce_allpairs, allreduce_ring
@@ -34,8 +34,9 @@ class Launcher:
 
     def __init__(self, comm, algo, check=True):
         from msccl.runtime.executor import MAX_SLOT_BYTES
-        from msccl.runtime.plan import K_FIFO_SLOTS, compile_plan, fifo_index_tables
-        self.comm, self.algo = comm, algo
+        from msccl.runtime.plan import K_FIFO_SLOTS, compile_plan, fifo_index_tables, occupy_idle_ranks
+        self.comm, self.algo = comm, occupy_idle_ranks(algo)
+        algo = self.algo
         conns = max(max(len(t) for t in fifo_index_tables(algo).values()), 1)
         self.slot = min(MAX_SLOT_BYTES, comm.fifo_bytes // (conns * K_FIFO_SLOTS)) // 1024 * 1024
         self.host = compile_plan(algo, comm.local_ranks, self.slot, check=check)
@@ -284,3 +285,27 @@ def test_adds_whose_source_is_refilled_between_them(emulated, protocol):
         assert torch.all(ins[0] == 1) and torch.all(ins[1] == 7)
     plan.close()
     run.close()
+
+
+@pytest.mark.parametrize('protocol', ['LL', 'LL128'])
+def test_a_rank_without_threadblocks_keeps_up(emulated, protocol):
+    """A program that leaves rank 2 idle, then one whose packet flags name the launch: every rank must have counted both."""
+    def pair():
+        chunk(1, Buffer.input, 0).reduce(chunk(0, Buffer.input, 0))
+    comm = emulated(3, 1 << 20)
+    comm.timeout_ns = int(2e9)
+    idle = _program('pair', AllReduce(3, 1, True), pair, protocol=protocol)
+    assert not idle.gpus[2].tbs
+    first = Launcher(comm, idle)
+    ring = Launcher(comm, _program('ring', AllReduce(3, 3, True), lambda: allreduce_ring(3, 1), 1,
+                                   threadblock_policy=ThreadblockPolicy.manual, protocol=protocol))
+    for _ in range(3):
+        ins = {r: torch.full((3 * 512,), float(r + 1), device='cuda') for r in range(3)}
+        first(ins)
+        comm.check()
+        assert [float(ins[r][5]) for r in range(3)] == [1, 3, 3]
+        ring(ins)
+        comm.check()
+        assert all(torch.all(ins[r] == 7) for r in range(3))
+    first.close()
+    ring.close()
